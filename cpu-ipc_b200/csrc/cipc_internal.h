@@ -235,7 +235,7 @@ struct Ctx {
     DBuf<float> mpGS, mpGD;
     DBuf<float> mpVec, mpDGS, mpDGD, mpDH, mpDES, mpDED, mpDAgg, mpDS, mpDSD;
     DBuf<float> mpBD, mpBX, mpPart;     // backward: per-item gradients, second input block, split-K partials
-    DBuf<unsigned char> mpLowS, mpLowD; // 1 for lower slots of the static / contact pattern
+    DBuf<int> mpEdgeOfS, mpEdgeOfD;     // a slot's place in the flat lists (-1: not a lower slot)
     DBuf<int> mpFlatS, mpFlatD;         // flat lower-edge lists: slot, row, column (3 arrays each, packed)
     int nFlatS = -1, nFlatD = 0;
     DBuf<int> mpScanTmpI;               // row counts and offsets of the flat lists

@@ -223,13 +223,13 @@ __global__ void __launch_bounds__(THREADS) denseTcKernel(int n, G gather, E emit
 // so that the two MMAs per K step carry d to about 16 bits and every product
 // is exact in the FP32 accumulator.  Each CTA accumulates its tiles in
 // tensor memory and writes one partial (OUT * 64 weights then OUT biases, the
-// layout of the CUDA-core kernel's partials); items with mask 0 contribute
-// nothing.  Dynamic shared memory: WG_SMEM bytes.  Waits are bounded as in
+// layout of the CUDA-core kernel's partials).  X1 is read at x1Item[item] (the
+// edge's slot) where that list is given.  Dynamic shared memory: WG_SMEM bytes.  Waits are bounded as in
 // denseTcKernel.
 constexpr int WG_K = 128;  // items per tile
 constexpr int WG_SMEM = M * WG_K * 2 + 2 * 32 * WG_K * 2;
 
-__global__ void __launch_bounds__(THREADS) weightGradTcKernel(int items, const float* D, const float* X1, const float* X2, const unsigned char* mask,
+__global__ void __launch_bounds__(THREADS) weightGradTcKernel(int items, const float* D, const float* X1, const int* x1Item, const float* X2,
                                                               float* partial, int* status, int timeoutBit) {
     constexpr int IN = 64, OUT = 32, NW = OUT * IN + OUT;
     extern __shared__ __align__(1024) unsigned char wgSmem[];
@@ -259,8 +259,8 @@ __global__ void __launch_bounds__(THREADS) weightGradTcKernel(int items, const f
     for (int base = blockIdx.x * WG_K; base < items; base += gridDim.x * WG_K) {
         // thread t stores item base + t as column t of A and of the two B terms
         const int it = base + tid;
-        const bool on = it < items && (!mask || mask[it]);
-        const float4* x1 = reinterpret_cast<const float4*>(X1 + (size_t)(on ? it : 0) * 32);
+        const bool on = it < items;
+        const float4* x1 = reinterpret_cast<const float4*>(X1 + (size_t)(on ? (x1Item ? x1Item[it] : it) : 0) * 32);
         const float4* x2 = reinterpret_cast<const float4*>(X2 + (size_t)(on ? it : 0) * 32);
 #pragma unroll
         for (int q = 0; q < 16; ++q) {

@@ -284,11 +284,15 @@ __global__ void lowerCountKernel(int nv, const int* rowS, const int* rowE, const
         cnt[v] = k;
     }
 }
-__global__ void lowerFillKernel(int nv, const int* rowS, const int* rowE, const int* col, const int* off, int* eSlot, int* eI, int* eJ) {
+// edgeOf[slot]: the lower slot's place in the list, -1 for the other slots
+__global__ void lowerFillKernel(int nv, const int* rowS, const int* rowE, const int* col, const int* off, int* eSlot, int* eI, int* eJ, int* edgeOf) {
     CIPC_KERNEL_LOOP(v, nv) {
         int o = off[v];
-        for (int s = rowS[v]; s < rowE[v]; ++s)
-            if (col[s] < v) { eSlot[o] = s; eI[o] = v; eJ[o] = col[s]; ++o; }
+        for (int s = rowS[v]; s < rowE[v]; ++s) {
+            const bool low = col[s] < v;
+            edgeOf[s] = low ? o : -1;
+            if (low) { eSlot[o] = s; eI[o] = v; eJ[o] = col[s]; ++o; }
+        }
     }
 }
 
@@ -386,12 +390,19 @@ struct HeadDiagEmit {
 };
 
 // ---------------------------------------------------------------------------
-// factor and scaled operator products (FP32 vectors, one thread per row)
+// factor and scaled operator products of all probe vectors at once (FP32
+// vectors, planes of 3 nv): one thread per row and probe, the probes of a row
+// in neighbouring lanes, so that a block is fetched once for all of them
+//
 // ---------------------------------------------------------------------------
 // y = G u (transpose = 0: lower slots + diagonal) or y = G^T u (mirror slots + transposed diagonal)
-__global__ void factorApplyKernel(int nv, int transpose, const int* rowPtr, const int* col, const float* gS, const int* dRowS, const int* dRowE,
-                                  const int* dCol, const float* gD, const float* u, float* y) {
-    CIPC_KERNEL_LOOP(v, nv) {
+__global__ void factorApplyKernel(int nv, int probes, int transpose, const int* rowPtr, const int* col, const float* gS, const int* dRowS, const int* dRowE,
+                                  const int* dCol, const float* gD, const float* uAll, float* yAll) {
+    CIPC_KERNEL_LOOP(i, nv * probes) {
+        const int v = i / probes;
+        const size_t plane = (size_t)(i - v * probes) * 3 * nv;
+        const float* u = uAll + plane;
+        float* y = yAll + plane;
         float acc[3] = {0.f, 0.f, 0.f};
         for (int k = rowPtr[v]; k < rowPtr[v + 1]; ++k) {
             int c = col[k];
@@ -417,9 +428,13 @@ __global__ void factorApplyKernel(int nv, int transpose, const int* rowPtr, cons
 
 // y = Â u = S A S^T u
 template <class MT>
-__global__ void scaledSpmvKernel(int nv, const int* rowPtr, const int* col, const MT* val, const int* dRowS, const int* dRowE, const int* dCol,
-                                 const MT* dVal, const double* diagExtra, const double* S, const float* u, float* y) {
-    CIPC_KERNEL_LOOP(v, nv) {
+__global__ void scaledSpmvKernel(int nv, int probes, const int* rowPtr, const int* col, const MT* val, const int* dRowS, const int* dRowE,
+                                 const int* dCol, const MT* dVal, const double* diagExtra, const double* S, const float* uAll, float* yAll) {
+    CIPC_KERNEL_LOOP(i, nv * probes) {
+        const int v = i / probes;
+        const size_t plane = (size_t)(i - v * probes) * 3 * nv;
+        const float* u = uAll + plane;
+        float* y = yAll + plane;
         double acc[3] = {0, 0, 0};
         auto stu = [&](int c, double x[3]) {
             // S_c^T u_c (S_c lower triangular)
@@ -468,8 +483,11 @@ __global__ void probeKernel(int n, unsigned long long seed, float* w) {
     }
 }
 
-// partials of u.v and w.w
-__global__ void probeDotsKernel(int n, const float* u, const float* v, const float* w, double* part) {
+// partials of u.v and w.w of probe blockIdx.y (planes of n)
+__global__ void probeDotsKernel(int n, const float* uAll, const float* vAll, const float* wAll, double* partAll) {
+    const size_t plane = (size_t)blockIdx.y * n;
+    const float *u = uAll + plane, *v = vAll + plane, *w = wAll + plane;
+    double* part = partAll + (size_t)2 * gridDim.x * blockIdx.y;
     double uv = 0, ww = 0;
     CIPC_KERNEL_LOOP(i, n) {
         uv += (double)u[i] * (double)v[i];
@@ -492,43 +510,51 @@ __global__ void logDiagKernel(int nv, const int* diagSlot, const float* gS, doub
     if (threadIdx.x == 0) part[blockIdx.x] = a;
 }
 
-// dG_ij += scale * w_i v_j^T for lower slots and the lower triangle of the
-// diagonal slot (static: dyn = 0); contact slots: lower only
-__global__ void factorGradKernel(int nv, const int* rowS, const int* rowE, const int* col, int dyn, const int* btype, const float* w, const float* vv,
-                                 float scale, float* dG) {
-    CIPC_KERNEL_LOOP(i, nv) {
-        if (btype[i] != 0) continue;
-        for (int k = rowS[i]; k < rowE[i]; ++k) {
-            int j = col[k];
-            if (j > i || (dyn && j == i) || btype[j] != 0) continue;
-            for (int a = 0; a < 3; ++a)
-                for (int b = 0; b < 3; ++b) {
-                    if (j == i && b > a) continue;
-                    dG[(size_t)9 * k + 3 * a + b] += scale * w[3 * i + a] * vv[3 * j + b];
-                }
-        }
+// The loss's gradient with respect to G, (1/T) sum over probes of
+// scale w_i v_j^T, a chunk of probes at a time (first: nothing is summed yet;
+// mul: 1/T with the last chunk, else 1): on the lower slots one thread per edge
+// and entry, the probes in their order, ...
+__global__ void factorGradEdgeKernel(int n, const int* slot, const int* ei, const int* ej, const int* btype, int probes, int n3, const float* w,
+                                     const float* vv, const float* scale, bool first, float mul, float* dG) {
+    CIPC_KERNEL_LOOP(t, 9 * n) {
+        const int e = t / 9, q = t - 9 * e, a = q / 3, b = q - 3 * a;
+        const int i = ei[e], j = ej[e];
+        float* o = dG + (size_t)9 * slot[e] + q;
+        float s = first ? 0.f : *o;
+        if (btype[i] == 0 && btype[j] == 0)
+            for (int p = 0; p < probes; ++p) s += scale[p] * w[(size_t)p * n3 + 3 * i + a] * vv[(size_t)p * n3 + 3 * j + b];
+        *o = s * mul;
     }
 }
-
-// dG /= T on the slots; on static diagonal slots also subtract (2/n) / G_qq
-__global__ void gradScaleKernel(size_t n, float invT, float* dG) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)blockDim.x * gridDim.x) dG[i] *= invT;
-}
-__global__ void gradDiagKernel(int nv, const int* diagSlot, const int* btype, const float* gS, float coef, float* dG) {
-    CIPC_KERNEL_LOOP(v, nv) {
-        if (btype[v] != 0) continue;
-        size_t s = (size_t)9 * diagSlot[v];
-        for (int q = 0; q < 3; ++q) dG[s + 4 * q] -= coef / gS[s + 4 * q];
+// ... and on the diagonal slots' lower triangles (zero above), where the log
+// term adds -(2/n) / G_qq on the free vertices.
+__global__ void factorGradDiagKernel(int nv, const int* diagSlot, const int* btype, int probes, int n3, const float* w, const float* vv,
+                                     const float* scale, bool first, float mul, bool last, const float* gS, float coef, float* dG) {
+    CIPC_KERNEL_LOOP(t, 9 * nv) {
+        const int v = t / 9, q = t - 9 * v, a = q / 3, b = q - 3 * a;
+        const size_t o = (size_t)9 * diagSlot[v] + q;
+        float s = first ? 0.f : dG[o];
+        if (btype[v] == 0 && b <= a) {
+            for (int p = 0; p < probes; ++p) s += scale[p] * w[(size_t)p * n3 + 3 * v + a] * vv[(size_t)p * n3 + 3 * v + b];
+            s *= mul;
+            if (last && a == b) s -= coef / gS[o];
+        }
+        dG[o] = s;
     }
 }
 
 // ---------------------------------------------------------------------------
 // backward
 //
-// Each layer's backward runs in two parts.  An item kernel (one thread per
-// node, or per row over its lower slots) forms the pre-activation gradient
-// d (written to D[item][OUT], zero for masked items) and propagates W^T d to
-// the layer's inputs.  The weight gradient dW = D^T X and db = sum D is then
+// Each layer's backward runs in two parts over items: nodes, or the edges of
+// the flat lower-edge lists (edge states of the forward pass are read at the
+// edge's slot, gradients are stored by edge).  An item kernel forms the
+// pre-activation gradient d (written to D[item][OUT]) and propagates W^T d to
+// the layer's inputs.  Every row of 32 values is read and written by 32
+// neighbouring lanes; one thread per matrix row walking its edges with
+// strided rows took most of an evaluation (loss and gradient, 4 probes, 8-cube
+// pile, 17,596 vertices: 5.68 -> 1.46 ms on a B200).  Bound now: launches of
+// 5-20 us each, the weight gradients among them.  The weight gradient dW = D^T X and db = sum D is then
 // a split-K reduction over the items: each CTA stages TI items of D and X in
 // shared memory and accumulates its share of the OUT x IN outputs in
 // registers, writes one partial per output, and a second kernel sums the
@@ -538,12 +564,13 @@ constexpr int WG_TI = 32;        // items per shared-memory tile
 constexpr int WG_THREADS = 256;
 constexpr int WG_GRID = 296;     // CTAs of the split-K reduction (2 per SM)
 
-// X = [X1 (ld1, IN1 columns) ; X2 (ld2, IN2 columns)] per item; mask may be
-// null (all items active).  partial[cta][OUT*(IN1+IN2) + OUT].  The heads
-// and the embeddings (the tensor-core layers use weightGradTcKernel).
+// X = [X1 (IN1 columns) ; X2 (IN2 columns)] per item; dItem and xItem are the
+// rows of D and of X1, X2 that belong to an item (null: the item's number).
+// partial[cta][OUT*(IN1+IN2) + OUT].  The heads and the embeddings (the
+// tensor-core layers use weightGradTcKernel).
 template <int OUT, int IN1, int IN2>
-__global__ void __launch_bounds__(WG_THREADS) weightGradKernel(int items, const float* D, const float* X1, const float* X2, const unsigned char* mask,
-                                                               float* partial) {
+__global__ void __launch_bounds__(WG_THREADS) weightGradKernel(int items, const float* D, const int* dItem, const float* X1, const float* X2,
+                                                               const int* xItem, float* partial) {
     constexpr int IN = IN1 + IN2;
     constexpr int NW = OUT * IN + OUT;
     constexpr int PER = (NW + WG_THREADS - 1) / WG_THREADS;
@@ -555,14 +582,15 @@ __global__ void __launch_bounds__(WG_THREADS) weightGradKernel(int items, const 
         __syncthreads();
         for (int t = threadIdx.x; t < WG_TI * OUT; t += WG_THREADS) {
             int it = base + t / OUT, o = t % OUT;
-            bool on = it < items && (!mask || mask[it]);
-            sD[t / OUT][o] = on ? D[(size_t)it * OUT + o] : 0.f;
+            sD[t / OUT][o] = it < items ? D[(size_t)(dItem ? dItem[it] : it) * OUT + o] : 0.f;
         }
         for (int t = threadIdx.x; t < WG_TI * IN; t += WG_THREADS) {
             int r = t / IN, i = t % IN, it = base + r;
-            bool on = it < items && (!mask || mask[it]);
             float v = 0.f;
-            if (on) v = i < IN1 ? X1[(size_t)it * IN1 + i] : X2[(size_t)it * IN2 + (i - IN1)];
+            if (it < items) {
+                const size_t row = xItem ? xItem[it] : it;
+                v = i < IN1 ? X1[row * IN1 + i] : X2[row * IN2 + (i - IN1)];
+            }
             sX[r][i] = v;
         }
         __syncthreads();
@@ -588,146 +616,172 @@ __global__ void __launch_bounds__(WG_THREADS) weightGradKernel(int items, const 
     }
 }
 
-// gW[w] += sum over CTAs of partial (weights at wOff, biases at bOff)
-__global__ void weightGradReduceKernel(int nw, int out, int ctas, const float* partial, float* gW, float* gB) {
-    CIPC_KERNEL_LOOP(idx, nw) {
-        float s = 0.f;
-        for (int g = 0; g < ctas; ++g) s += partial[(size_t)g * nw + idx];
+// gW[w] += sum over CTAs of partial (weights, then `out` biases).  WR_SPLIT
+// threads share a weight, each adds every WR_SPLIT-th CTA, and their sums are
+// added in a fixed order: a thread that read all 296 partials one after the
+// other took 33 us.
+constexpr int WR_OUT = 32, WR_SPLIT = 8;
+__global__ void __launch_bounds__(WR_OUT * WR_SPLIT) weightGradReduceKernel(int nw, int out, int ctas, const float* partial, float* gW, float* gB) {
+    __shared__ float sh[WR_SPLIT][WR_OUT];
+    const int o = threadIdx.x % WR_OUT, part = threadIdx.x / WR_OUT, idx = blockIdx.x * WR_OUT + o;
+    float s = 0.f;
+    if (idx < nw)
+        for (int g = part; g < ctas; g += WR_SPLIT) s += partial[(size_t)g * nw + idx];
+    sh[part][o] = s;
+    __syncthreads();
+    if (part == 0 && idx < nw) {
+        for (int k = 1; k < WR_SPLIT; ++k) s += sh[k][o];
         if (idx < nw - out) gW[idx] += s;
         else gB[idx - (nw - out)] += s;
     }
 }
 
+// one warp per node: lane t forms component t of W^T d
 __global__ void headDiagBackKernel(int nv, const float* headD, const int* diagSlot, const float* dGS, const bf16* w, float* D6, float* dhL) {
-    CIPC_KERNEL_LOOP(v, nv) {
+    const int lane = threadIdx.x & 31, warps = gridDim.x * blockDim.x / 32;
+    float wt[6];
+    for (int q = 0; q < 6; ++q) wt[q] = W(w + MP_WD, q * MPNN_H + lane);
+    for (int v = (blockIdx.x * blockDim.x + threadIdx.x) / 32; v < nv; v += warps) {
         const float* dB = dGS + (size_t)9 * diagSlot[v];
-        const float* o = headD + 6 * v;
-        float d[6] = {dB[0] * sigmoidf(o[0]), dB[4] * sigmoidf(o[1]), dB[8] * sigmoidf(o[2]), dB[3], dB[6], dB[7]};
-        float dh[MPNN_H];
-        for (int t = 0; t < MPNN_H; ++t) dh[t] = 0.f;
-        for (int q = 0; q < 6; ++q) {
-            D6[6 * v + q] = d[q];
-            for (int t = 0; t < MPNN_H; ++t) dh[t] += d[q] * W(w + MP_WD, q * MPNN_H + t);
-        }
-        for (int t = 0; t < MPNN_H; ++t) dhL[(size_t)MPNN_H * v + t] = dh[t];
+        const float* o = headD + 6 * (size_t)v;
+        const float d[6] = {dB[0] * sigmoidf(o[0]), dB[4] * sigmoidf(o[1]), dB[8] * sigmoidf(o[2]), dB[3], dB[6], dB[7]};
+        float dh = 0.f;
+        for (int q = 0; q < 6; ++q) dh += d[q] * wt[q];
+        float mine = d[0];
+        for (int q = 1; q < 6; ++q) mine = lane == q ? d[q] : mine;
+        if (lane < 6) D6[6 * (size_t)v + lane] = mine;
+        dhL[(size_t)MPNN_H * v + lane] = dh;
     }
 }
 
-__global__ void headEdgeBackKernel(int nv, const int* rowS, const int* rowE, const int* col, const float* dG, const bf16* w, float* D9, float* deL) {
+// one warp per edge (its output gradient is the edge's block of dG)
+__global__ void headEdgeBackKernel(int n, const int* slot, const float* dG, const bf16* w, float* deL) {
     constexpr int IN = MPNN_H + MPNN_EF;
-    CIPC_KERNEL_LOOP(v, nv) {
-        for (int k = rowS[v]; k < rowE[v]; ++k) {
-            if (col[k] >= v) continue;
-            const float* d = dG + (size_t)9 * k;
-            float dh[MPNN_H];
-            for (int t = 0; t < MPNN_H; ++t) dh[t] = 0.f;
-            for (int q = 0; q < 9; ++q) {
-                D9[(size_t)9 * k + q] = d[q];
-                const bf16* Wr = w + MP_WO + q * IN;
-                for (int t = 0; t < MPNN_H; ++t) dh[t] += d[q] * W(Wr, t);
+    const int lane = threadIdx.x & 31, warps = gridDim.x * blockDim.x / 32;
+    float wt[9];
+    for (int q = 0; q < 9; ++q) wt[q] = W(w + MP_WO + q * IN, lane);
+    for (int e = (blockIdx.x * blockDim.x + threadIdx.x) / 32; e < n; e += warps) {
+        const float* d = dG + (size_t)9 * slot[e];
+        float dh = 0.f;
+        for (int q = 0; q < 9; ++q) dh += d[q] * wt[q];
+        deL[(size_t)MPNN_H * e + lane] = dh;
+    }
+}
+
+// Backward of a 64 -> 32 layer over tiles of LB_ITEMS items: the warps form the
+// items' pre-activation gradients d (one row of 32 per warp step; also kept in
+// shared memory), then two threads per item each form 32 of the 64 components
+// of W^T d from the staged weights.
+constexpr int LB_ITEMS = 64, LB_THREADS = 2 * LB_ITEMS;
+
+struct NodeBack {  // h' = relu(Wh [h; agg] + b)
+    const float *hNext, *dhNext;
+    float *dhPrev, *dagg;
+    __device__ float pre(int v, int t) const { return hNext[(size_t)MPNN_H * v + t] > 0.f ? dhNext[(size_t)MPNN_H * v + t] : 0.f; }
+    __device__ float* out(int v, int half) const { return (half ? dagg : dhPrev) + (size_t)MPNN_H * v; }
+};
+// e' = relu(We [e; h_i + h_j] + b); the edge's gradient is deNext plus what the
+// node layer's mean takes from it, dagg_i / deg_i + dagg_j / deg_j.  Writes the
+// gradient with respect to e (dePrev) and to h_i + h_j (ds), and that sum (the
+// second input block of the weight gradient).
+struct EdgeBack {
+    const int *slot, *ei, *ej;
+    const float *hPrev, *eNext, *deNext, *dagg;
+    const int* deg;
+    float *hsum, *dePrev, *ds;
+    __device__ float pre(int k, int t) const {
+        const int i = ei[k], j = ej[k];
+        hsum[(size_t)MPNN_H * k + t] = hPrev[(size_t)MPNN_H * i + t] + hPrev[(size_t)MPNN_H * j + t];
+        const float iv = deg[i] > 0 ? 1.f / deg[i] : 0.f, ic = deg[j] > 0 ? 1.f / deg[j] : 0.f;
+        const float de = deNext[(size_t)MPNN_H * k + t] + (dagg[(size_t)MPNN_H * i + t] * iv + dagg[(size_t)MPNN_H * j + t] * ic);
+        return eNext[(size_t)MPNN_H * slot[k] + t] > 0.f ? de : 0.f;
+    }
+    __device__ float* out(int k, int half) const { return (half ? ds : dePrev) + (size_t)MPNN_H * k; }
+};
+
+template <class B>
+__global__ void __launch_bounds__(LB_THREADS) layerBackKernel(int n, B b, const bf16* Wm, float* D32) {
+    __shared__ __align__(16) float sW[MPNN_H][2 * MPNN_H];
+    __shared__ float sD[LB_ITEMS][MPNN_H + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int t = threadIdx.x; t < MPNN_H * 2 * MPNN_H; t += LB_THREADS) sW[t / (2 * MPNN_H)][t % (2 * MPNN_H)] = W(Wm, t);
+    for (int base = blockIdx.x * LB_ITEMS; base < n; base += gridDim.x * LB_ITEMS) {
+        __syncthreads();
+        for (int r = warp; r < LB_ITEMS; r += LB_THREADS / 32) {
+            const int item = base + r;
+            float d = 0.f;
+            if (item < n) {
+                d = b.pre(item, lane);
+                D32[(size_t)MPNN_H * item + lane] = d;
             }
-            for (int t = 0; t < MPNN_H; ++t) deL[(size_t)MPNN_H * k + t] = dh[t];
+            sD[r][lane] = d;
         }
-    }
-}
-
-// node layer backward: h' = relu(Wh [h; agg] + b)
-__global__ void nodeLayerBackKernel(int nv, const float* hNext, const float* dhNext, const bf16* Wm, float* D32, float* dhPrev, float* dagg) {
-    CIPC_KERNEL_LOOP(v, nv) {
-        float dpre[MPNN_H];
-        for (int t = 0; t < MPNN_H; ++t) {
-            dpre[t] = hNext[(size_t)MPNN_H * v + t] > 0.f ? dhNext[(size_t)MPNN_H * v + t] : 0.f;
-            D32[(size_t)MPNN_H * v + t] = dpre[t];
-        }
-        for (int i = 0; i < 2 * MPNN_H; ++i) {
-            float s = 0.f;
-            for (int o = 0; o < MPNN_H; ++o) s += W(Wm, o * 2 * MPNN_H + i) * dpre[o];
-            if (i < MPNN_H) dhPrev[(size_t)MPNN_H * v + i] += s;
-            else dagg[(size_t)MPNN_H * v + i - MPNN_H] = s;
-        }
-    }
-}
-
-// d e_k += dagg_i / deg_i + dagg_j / deg_j for the edge k = (i, j)
-__global__ void aggBackKernel(int nv, const int* rowS, const int* rowE, const int* col, const float* dagg, const int* deg, float* de) {
-    CIPC_KERNEL_LOOP(v, nv) {
-        for (int k = rowS[v]; k < rowE[v]; ++k) {
-            int c = col[k];
-            if (c >= v) continue;
-            float iv = deg[v] > 0 ? 1.f / deg[v] : 0.f, ic = deg[c] > 0 ? 1.f / deg[c] : 0.f;
-            for (int t = 0; t < MPNN_H; ++t) de[(size_t)MPNN_H * k + t] += dagg[(size_t)MPNN_H * v + t] * iv + dagg[(size_t)MPNN_H * c + t] * ic;
-        }
-    }
-}
-
-// edge layer backward: e' = relu(We [e; h_i + h_j] + b); adds to de^l,
-// writes ds_k (the gradient with respect to h_i + h_j), the pre-activation
-// gradient and the summed endpoint states (the second input block)
-__global__ void edgeLayerBackKernel(int nv, const int* rowS, const int* rowE, const int* col, const float* hPrev, const float* eNext,
-                                    const float* deNext, const bf16* Wm, float* D32, float* hsum, float* dePrev, float* ds) {
-    CIPC_KERNEL_LOOP(v, nv) {
-        for (int k = rowS[v]; k < rowE[v]; ++k) {
-            int c = col[k];
-            if (c >= v) continue;
-            float dpre[MPNN_H];
-            for (int t = 0; t < MPNN_H; ++t) {
-                dpre[t] = eNext[(size_t)MPNN_H * k + t] > 0.f ? deNext[(size_t)MPNN_H * k + t] : 0.f;
-                D32[(size_t)MPNN_H * k + t] = dpre[t];
-                hsum[(size_t)MPNN_H * k + t] = hPrev[(size_t)MPNN_H * v + t] + hPrev[(size_t)MPNN_H * c + t];
-            }
-            for (int i = 0; i < 2 * MPNN_H; ++i) {
-                float s = 0.f;
-                for (int o = 0; o < MPNN_H; ++o) s += W(Wm, o * 2 * MPNN_H + i) * dpre[o];
-                if (i < MPNN_H) dePrev[(size_t)MPNN_H * k + i] += s;
-                else ds[(size_t)MPNN_H * k + i - MPNN_H] = s;
+        __syncthreads();
+        // lanes 0-15 of a warp take 16 items' first halves, 16-31 the second
+        const int r = 16 * warp + (lane & 15), half = lane >> 4, item = base + r;
+        float acc[MPNN_H];
+#pragma unroll
+        for (int i = 0; i < MPNN_H; ++i) acc[i] = 0.f;
+#pragma unroll 4
+        for (int o = 0; o < MPNN_H; ++o) {
+            const float d = sD[r][o];
+            const float4* wr = reinterpret_cast<const float4*>(&sW[o][half * MPNN_H]);
+#pragma unroll
+            for (int i = 0; i < MPNN_H / 4; ++i) {
+                const float4 w4 = wr[i];
+                acc[4 * i] += w4.x * d;
+                acc[4 * i + 1] += w4.y * d;
+                acc[4 * i + 2] += w4.z * d;
+                acc[4 * i + 3] += w4.w * d;
             }
         }
-    }
-}
-
-// dh_v += sum of ds over the edges incident to v (read at their lower slot)
-__global__ void dsGatherKernel(int nv, const int* rowPtr, const int* col, const int* mirS, const float* dsS, const int* dRowS, const int* dRowE,
-                               const int* dCol, const int* mirD, const float* dsD, float* dh) {
-    CIPC_KERNEL_LOOP(v, nv) {
-        float s[MPNN_H];
-        for (int t = 0; t < MPNN_H; ++t) s[t] = 0.f;
-        for (int k = rowPtr[v]; k < rowPtr[v + 1]; ++k) {
-            int c = col[k];
-            if (c == v) continue;
-            int slot = c < v ? k : mirS[k];
-            if (slot < 0) continue;
-            for (int t = 0; t < MPNN_H; ++t) s[t] += dsS[(size_t)MPNN_H * slot + t];
-        }
-        if (dRowS)
-            for (int k = dRowS[v]; k < dRowE[v]; ++k) {
-                int c = dCol[k];
-                if (c == v) continue;
-                int slot = c < v ? k : mirD[k];
-                if (slot < 0) continue;
-                for (int t = 0; t < MPNN_H; ++t) s[t] += dsD[(size_t)MPNN_H * slot + t];
-            }
-        for (int t = 0; t < MPNN_H; ++t) dh[(size_t)MPNN_H * v + t] += s[t];
-    }
-}
-
-// pre-activation gradient of an embedding (relu): items are nodes or, with
-// row ranges, the lower slots of a pattern
-__global__ void reluGradNodeKernel(int nv, const float* y, const float* dy, float* D32) {
-    CIPC_KERNEL_LOOP(i, nv * MPNN_H) D32[i] = y[i] > 0.f ? dy[i] : 0.f;
-}
-__global__ void reluGradEdgeKernel(int nv, const int* rowS, const int* rowE, const int* col, const float* y, const float* dy, float* D32) {
-    CIPC_KERNEL_LOOP(v, nv) {
-        for (int k = rowS[v]; k < rowE[v]; ++k) {
-            if (col[k] >= v) continue;
-            for (int t = 0; t < MPNN_H; ++t) D32[(size_t)MPNN_H * k + t] = y[(size_t)MPNN_H * k + t] > 0.f ? dy[(size_t)MPNN_H * k + t] : 0.f;
+        if (item < n) {
+            float4* out = reinterpret_cast<float4*>(b.out(item, half));
+#pragma unroll
+            for (int i = 0; i < MPNN_H / 4; ++i) out[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
         }
     }
 }
 
-// 1 for lower slots (col < row) of a row-ranged pattern, else 0
-__global__ void lowerMaskKernel(int nv, const int* rowS, const int* rowE, const int* col, unsigned char* mask) {
-    CIPC_KERNEL_LOOP(v, nv) {
-        for (int k = rowS[v]; k < rowE[v]; ++k) mask[k] = col[k] < v ? 1 : 0;
+// sum over the row's edges of feature `lane` of e, slot order (as
+// aggregateRange, rows by edge)
+__device__ __forceinline__ float edgeSumRange(float a, int v, int k0, int k1, const int* col, const int* mir, const int* edgeOf, const float* e,
+                                              int lane) {
+    for (int c0 = k0; c0 < k1; c0 += 32) {
+        const int k = c0 + lane;
+        int edge = -1;
+        if (k < k1) {
+            const int c = col[k];
+            const int slot = c == v ? -1 : (c < v ? k : mir[k]);
+            if (slot >= 0) edge = edgeOf[slot];
+        }
+        const int m = min(32, k1 - c0);
+        for (int j = 0; j < m; ++j) {
+            const int ej = __shfl_sync(0xffffffffu, edge, j);
+            if (ej >= 0) a += e[(size_t)MPNN_H * ej + lane];
+        }
+    }
+    return a;
+}
+
+// dh_v += sum of ds over the edges incident to v, one warp per vertex
+__global__ void dsGatherKernel(int nv, const int* rowPtr, const int* col, const int* mirS, const int* edgeS, const float* dsS, const int* dRowS,
+                               const int* dRowE, const int* dCol, const int* mirD, const int* edgeD, const float* dsD, float* dh) {
+    const int lane = threadIdx.x & 31;
+    const int warps = gridDim.x * blockDim.x / 32;
+    for (int v = (blockIdx.x * blockDim.x + threadIdx.x) / 32; v < nv; v += warps) {
+        float s = edgeSumRange(0.f, v, rowPtr[v], rowPtr[v + 1], col, mirS, edgeS, dsS, lane);
+        if (dRowS) s = edgeSumRange(s, v, dRowS[v], dRowE[v], dCol, mirD, edgeD, dsD, lane);
+        dh[(size_t)MPNN_H * v + lane] += s;
+    }
+}
+
+// pre-activation gradient of an embedding (relu): items are nodes or edges,
+// whose forward state is at their slot
+__global__ void reluGradKernel(int n, const int* slot, const float* y, const float* dy, float* D32) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n * MPNN_H; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t item = i / MPNN_H, t = i - item * MPNN_H;
+        D32[i] = y[(slot ? (size_t)slot[item] : item) * MPNN_H + t] > 0.f ? dy[i] : 0.f;
     }
 }
 
@@ -821,8 +875,9 @@ void mpnnGetGrad(Ctx& c, float* g) {
 }
 
 // Flat list of the lower edges of a row-ranged pattern: three arrays of
-// `count` ints (slot, row, column) packed in `out`.  Returns the count.
-static int buildLowerList(Ctx& c, const int* rowS, const int* rowE, const int* col, DBuf<int>& out) {
+// `count` ints (slot, row, column) packed in `out`, and each slot's place in
+// it (edgeOf, -1 for the other slots).  Returns the count.
+static int buildLowerList(Ctx& c, const int* rowS, const int* rowE, const int* col, DBuf<int>& out, int* edgeOf) {
     int nv = c.nv;
     c.mpScanTmpI.reserve(2 * (size_t)nv + 2);
     int* cnt = c.mpScanTmpI.p;
@@ -837,7 +892,7 @@ static int buildLowerList(Ctx& c, const int* rowS, const int* rowE, const int* c
     CIPC_CUDA(cudaMemcpyAsync(&n, off + nv, sizeof(int), cudaMemcpyDeviceToHost, c.s));
     hostSync(c);
     out.reserve(3 * (size_t)std::max(n, 1));
-    if (n > 0) launch(lowerFillKernel, blocksFor(nv), TB, 0, c.s, nv, rowS, rowE, col, (const int*)off, out.p, out.p + n, out.p + 2 * (size_t)n);
+    launch(lowerFillKernel, blocksFor(nv), TB, 0, c.s, nv, rowS, rowE, col, (const int*)off, out.p, out.p + n, out.p + 2 * (size_t)n, edgeOf);
     return n;
 }
 
@@ -859,8 +914,6 @@ static void prepareT(Ctx& c, const MT* val, const MT* dval, bool features) {
         c.mpRowS.reserve(nv); c.mpRowE.reserve(nv);
         launch(rowRangeKernel, blocksFor(nv), TB, 0, c.s, nv, (const int*)c.rowPtr.p, c.mpRowS.p, c.mpRowE.p);
         launch(mirrorKernel, blocksFor(nv), TB, 0, c.s, nv, (const int*)c.mpRowS.p, (const int*)c.mpRowE.p, (const int*)c.colIdx.p, c.mpMirS.p);
-        c.mpLowS.reserve(es);
-        launch(lowerMaskKernel, blocksFor(nv), TB, 0, c.s, nv, (const int*)c.mpRowS.p, (const int*)c.mpRowE.p, (const int*)c.colIdx.p, c.mpLowS.p);
         c.mpMirrorReady = true;
     }
     c.mpEdgeF.reserve(9 * es);
@@ -869,15 +922,17 @@ static void prepareT(Ctx& c, const MT* val, const MT* dval, bool features) {
                (const double*)c.mpS.p, c.mpEdgeF.p);
     c.mpMirD.reserve(ed);
     c.mpEdgeFD.reserve(9 * ed);
-    c.mpLowD.reserve(ed);
     if (d.on) {
         launch(mirrorKernel, blocksFor(nv), TB, 0, c.s, nv, d.rs, d.re, d.col, c.mpMirD.p);
-        launch(lowerMaskKernel, blocksFor(nv), TB, 0, c.s, nv, d.rs, d.re, d.col, c.mpLowD.p);
         if (features) launch(edgeFeatKernel<MT>, blocksFor(nv), TB, 0, c.s, nv, d.rs, d.re, d.col, dval, (const double*)c.mpS.p, c.mpEdgeFD.p);
     }
     if (features) {  // the network's flat edge lists
-        if (c.nFlatS < 0) c.nFlatS = buildLowerList(c, (const int*)c.mpRowS.p, (const int*)c.mpRowE.p, (const int*)c.colIdx.p, c.mpFlatS);
-        c.nFlatD = d.on ? buildLowerList(c, d.rs, d.re, d.col, c.mpFlatD) : 0;
+        if (c.nFlatS < 0) {
+            c.mpEdgeOfS.reserve(es);
+            c.nFlatS = buildLowerList(c, (const int*)c.mpRowS.p, (const int*)c.mpRowE.p, (const int*)c.colIdx.p, c.mpFlatS, c.mpEdgeOfS.p);
+        }
+        c.mpEdgeOfD.reserve(ed);
+        c.nFlatD = d.on ? buildLowerList(c, d.rs, d.re, d.col, c.mpFlatD, c.mpEdgeOfD.p) : 0;
     }
     c.mpDeg.reserve(nv);
     launch(degreeKernel, blocksFor(nv), TB, 0, c.s, nv, (const int*)c.rowPtr.p, (const int*)c.colIdx.p, (const int*)c.mpMirS.p, d.rs, d.re, d.col,
@@ -952,44 +1007,61 @@ static double lossT(Ctx& c, const MT* val, const MT* dval, int nprobes, const fl
     int nv = c.nv, n3 = 3 * nv;
     DynView d = dynView(c);
     size_t es = (size_t)std::max(c.nnzb, 1), ed = (size_t)std::max(c.nDynB, 1);
-    c.mpVec.reserve(3 * (size_t)n3);
+    // probes in chunks: planes of 3 nv per probe of w, u = G^T w, v = Â G^T w; then the scales
+    constexpr int CHUNK = 8;
+    const int chunk = std::min(nprobes, CHUNK);
+    const size_t np3 = (size_t)chunk * n3;
+    c.mpVec.reserve(3 * np3 + chunk);
     float* w = c.mpVec.p;
-    float* u = w + n3;   // G^T w
-    float* vv = u + n3;  // Â G^T w
+    float* u = w + np3;
+    float* vv = u + np3;
+    float* scaleDev = vv + np3;
+    const int nb = std::min(1024, std::max(1, (n3 + 255) / 256));
+    c.red.reserve(2 * 1024 * CHUNK + 16);
+    std::vector<double> part(std::max<size_t>(2 * (size_t)nb * chunk, 1024));
+    float scale[CHUNK];
+    const int nS = c.nFlatS, nE = d.on ? c.nFlatD : 0;
+    const int *sSlot = c.mpFlatS.p, *sI = sSlot + nS, *sJ = sSlot + 2 * (size_t)nS;
+    const int *dSlot = c.mpFlatD.p, *dI = dSlot + nE, *dJ = dSlot + 2 * (size_t)nE;
     if (backward) {
         c.mpDGS.reserve(9 * es);
         c.mpDGD.reserve(9 * ed);
-        zeroF(c, c.mpDGS.p, 9 * es);
-        zeroF(c, c.mpDGD.p, 9 * ed);
     }
-    int nb = std::min(1024, std::max(1, (n3 + 255) / 256));
-    c.red.reserve(2 * 1024 + 16);
-    std::vector<double> part(2 * nb + 2 * 1024);
     double T = 0;
-    for (int pr = 0; pr < nprobes; ++pr) {
+    for (int p0 = 0; p0 < nprobes; p0 += chunk) {
+        const int np = std::min(chunk, nprobes - p0);
         if (hostProbes)
-            CIPC_CUDA(cudaMemcpyAsync(w, hostProbes + (size_t)pr * n3, sizeof(float) * n3, cudaMemcpyHostToDevice, c.s));
+            CIPC_CUDA(cudaMemcpyAsync(w, hostProbes + (size_t)p0 * n3, sizeof(float) * n3 * np, cudaMemcpyHostToDevice, c.s));
         else
-            launch(probeKernel, blocksFor(n3), TB, 0, c.s, n3, seed + 7919ull * pr, w);
-        launch(factorApplyKernel, blocksFor(nv), TB, 0, c.s, nv, 1, (const int*)c.rowPtr.p, (const int*)c.colIdx.p, (const float*)c.mpGS.p, d.rs, d.re,
-               d.col, (const float*)c.mpGD.p, (const float*)w, u);
-        launch(scaledSpmvKernel<MT>, blocksFor(nv), TB, 0, c.s, nv, (const int*)c.rowPtr.p, (const int*)c.colIdx.p, val, d.rs, d.re, d.col, dval,
-               (const double*)c.diagExtra.p, (const double*)c.mpS.p, (const float*)u, vv);
-        launch(probeDotsKernel, nb, 256, 0, c.s, n3, (const float*)u, (const float*)vv, (const float*)w, c.red.p);
-        CIPC_CUDA(cudaMemcpyAsync(part.data(), c.red.p, sizeof(double) * 2 * nb, cudaMemcpyDeviceToHost, c.s));
+            for (int k = 0; k < np; ++k)
+                launch(probeKernel, blocksFor(n3), TB, 0, c.s, n3, seed + 7919ull * (p0 + k), w + (size_t)k * n3);
+        launch(factorApplyKernel, blocksFor(nv * np), TB, 0, c.s, nv, np, 1, (const int*)c.rowPtr.p, (const int*)c.colIdx.p, (const float*)c.mpGS.p,
+               d.rs, d.re, d.col, (const float*)c.mpGD.p, (const float*)w, u);
+        launch(scaledSpmvKernel<MT>, blocksFor(nv * np), TB, 0, c.s, nv, np, (const int*)c.rowPtr.p, (const int*)c.colIdx.p, val, d.rs, d.re, d.col,
+               dval, (const double*)c.diagExtra.p, (const double*)c.mpS.p, (const float*)u, vv);
+        launch(probeDotsKernel, dim3(nb, np), 256, 0, c.s, n3, (const float*)u, (const float*)vv, (const float*)w, c.red.p);
+        CIPC_CUDA(cudaMemcpyAsync(part.data(), c.red.p, sizeof(double) * 2 * nb * np, cudaMemcpyDeviceToHost, c.s));
         hostSync(c);
-        double uv = 0, ww = 0;
-        for (int k = 0; k < nb; ++k) { uv += part[2 * k]; ww += part[2 * k + 1]; }
-        if (!(ww > 0)) throw InvalidArgument("probe vector is zero");
-        T += uv / ww / nprobes;
-        if (backward) {
-            float scale = (float)(2.0 / ww / nprobes);
-            launch(factorGradKernel, blocksFor(nv), TB, 0, c.s, nv, (const int*)c.mpRowS.p, (const int*)c.mpRowE.p, (const int*)c.colIdx.p, 0,
-                   (const int*)c.btype.p, (const float*)w, (const float*)vv, scale, c.mpDGS.p);
-            if (d.on)
-                launch(factorGradKernel, blocksFor(nv), TB, 0, c.s, nv, d.rs, d.re, d.col, 1, (const int*)c.btype.p, (const float*)w, (const float*)vv,
-                       scale, c.mpDGD.p);
+        for (int k = 0; k < np; ++k) {
+            const double* pp = part.data() + (size_t)2 * nb * k;
+            double uv = 0, ww = 0;
+            for (int q = 0; q < nb; ++q) { uv += pp[2 * q]; ww += pp[2 * q + 1]; }
+            if (!(ww > 0)) throw InvalidArgument("probe vector is zero");
+            T += uv / ww / nprobes;
+            scale[k] = (float)(2.0 / ww / nprobes);
         }
+        if (!backward) continue;
+        const bool first = p0 == 0, last = p0 + np >= nprobes;
+        const float mul = last ? (float)(1.0 / T) : 1.f;
+        CIPC_CUDA(cudaMemcpyAsync(scaleDev, scale, sizeof(float) * np, cudaMemcpyHostToDevice, c.s));
+        if (nS)
+            launch(factorGradEdgeKernel, blocksFor(9 * nS), TB, 0, c.s, nS, sSlot, sI, sJ, (const int*)c.btype.p, np, n3, (const float*)w,
+                   (const float*)vv, (const float*)scaleDev, first, mul, c.mpDGS.p);
+        if (nE)
+            launch(factorGradEdgeKernel, blocksFor(9 * nE), TB, 0, c.s, nE, dSlot, dI, dJ, (const int*)c.btype.p, np, n3, (const float*)w,
+                   (const float*)vv, (const float*)scaleDev, first, mul, c.mpDGD.p);
+        launch(factorGradDiagKernel, blocksFor(9 * nv), TB, 0, c.s, nv, (const int*)c.diagSlot.p, (const int*)c.btype.p, np, n3, (const float*)w,
+               (const float*)vv, (const float*)scaleDev, first, mul, last, (const float*)c.mpGS.p, (float)(2.0 / n3), c.mpDGS.p);
     }
     int nb2 = std::min(1024, std::max(1, (nv + 255) / 256));
     launch(logDiagKernel, nb2, 256, 0, c.s, nv, (const int*)c.diagSlot.p, (const float*)c.mpGS.p, c.red.p);
@@ -1001,46 +1073,43 @@ static double lossT(Ctx& c, const MT* val, const MT* dval, int nprobes, const fl
     double loss = std::log(T) - 2.0 / n3 * logDiag;
     if (!backward) return loss;
 
-    launch(gradScaleKernel, 1024, 256, 0, c.s, 9 * es, (float)(1.0 / T), c.mpDGS.p);
-    if (d.on) launch(gradScaleKernel, 1024, 256, 0, c.s, 9 * ed, (float)(1.0 / T), c.mpDGD.p);
-    launch(gradDiagKernel, blocksFor(nv), TB, 0, c.s, nv, (const int*)c.diagSlot.p, (const int*)c.btype.p, (const float*)c.mpGS.p, (float)(2.0 / n3),
-           c.mpDGS.p);
-
     const bf16* wb = wbf(c);
     float* gW = c.mpG.p;
     zeroF(c, gW, MP_NPARAM);
-    size_t items = std::max(std::max(es, ed), (size_t)nv);
+    const size_t fS = (size_t)std::max(nS, 1), fD = (size_t)std::max(nE, 1);
+    size_t items = std::max(std::max(fS, fD), (size_t)nv);
     c.mpDH.reserve((size_t)(MPNN_L + 1) * MPNN_H * nv);
-    c.mpDES.reserve((size_t)(MPNN_L + 1) * MPNN_H * es);
-    c.mpDED.reserve((size_t)(MPNN_L + 1) * MPNN_H * ed);
+    c.mpDES.reserve((size_t)(MPNN_L + 1) * MPNN_H * fS);
+    c.mpDED.reserve((size_t)(MPNN_L + 1) * MPNN_H * fD);
     c.mpDAgg.reserve((size_t)MPNN_H * nv);
-    c.mpDS.reserve((size_t)MPNN_H * es);
-    c.mpDSD.reserve((size_t)MPNN_H * ed);
+    c.mpDS.reserve((size_t)MPNN_H * fS);
+    c.mpDSD.reserve((size_t)MPNN_H * fD);
     c.mpBD.reserve((size_t)MPNN_H * items);
     c.mpBX.reserve((size_t)MPNN_H * items);
     c.mpPart.reserve((size_t)WG_GRID * (MPNN_H * 2 * MPNN_H + MPNN_H));
-    zeroF(c, c.mpDH.p, (size_t)(MPNN_L + 1) * MPNN_H * nv);
-    zeroF(c, c.mpDES.p, (size_t)(MPNN_L + 1) * MPNN_H * es);
-    zeroF(c, c.mpDED.p, (size_t)(MPNN_L + 1) * MPNN_H * ed);
     auto H = [&](int l) { return c.mpH.p + (size_t)l * MPNN_H * nv; };
     auto DH = [&](int l) { return c.mpDH.p + (size_t)l * MPNN_H * nv; };
     auto ES = [&](int l) { return c.mpES.p + (size_t)l * MPNN_H * es; };
     auto ED = [&](int l) { return c.mpED.p + (size_t)l * MPNN_H * ed; };
-    auto DES = [&](int l) { return c.mpDES.p + (size_t)l * MPNN_H * es; };
-    auto DED = [&](int l) { return c.mpDED.p + (size_t)l * MPNN_H * ed; };
-    const int *rs = c.mpRowS.p, *re = c.mpRowE.p, *col = c.colIdx.p;
+    auto DES = [&](int l) { return c.mpDES.p + (size_t)l * MPNN_H * fS; };
+    auto DED = [&](int l) { return c.mpDED.p + (size_t)l * MPNN_H * fD; };
     float* BD = c.mpBD.p;
     float* BX = c.mpBX.p;
+    auto reduceWeights = [&](int nw, int out, int ctas, int wOff, int bOff) {
+        launch(weightGradReduceKernel, (nw + WR_OUT - 1) / WR_OUT, WR_OUT * WR_SPLIT, 0, c.s, nw, out, ctas, (const float*)c.mpPart.p, gW + wOff,
+               gW + bOff);
+    };
     // dW += D^T [X1 X2], db += sum D over `n` items (split-K, deterministic)
-    auto wgrad = [&](auto kernel, int out, int in, int n, const float* X1, const float* X2, const unsigned char* mask, int wOff, int bOff) {
+    auto wgrad = [&](auto kernel, int out, int in, int n, const float* D, const int* dItem, const float* X1, const float* X2, const int* xItem,
+                     int wOff, int bOff) {
         if (n <= 0) return;
         int nw = out * in + out;
         int grid = std::max(1, std::min(WG_GRID, (n + WG_TI - 1) / WG_TI));
-        launch(kernel, grid, WG_THREADS, 0, c.s, n, (const float*)BD, X1, X2, mask, c.mpPart.p);
-        launch(weightGradReduceKernel, blocksFor(nw), TB, 0, c.s, nw, out, grid, (const float*)c.mpPart.p, gW + wOff, gW + bOff);
+        launch(kernel, grid, WG_THREADS, 0, c.s, n, D, dItem, X1, X2, xItem, c.mpPart.p);
+        reduceWeights(nw, out, grid, wOff, bOff);
     };
     // the 64 -> 32 message-passing layers: the same contraction on the tensor cores
-    auto wgradTc = [&](int n, const float* X1, const float* X2, const unsigned char* mask, int wOff, int bOff) {
+    auto wgradTc = [&](int n, const float* X1, const int* x1Item, const float* X2, int wOff, int bOff) {
         if (n <= 0) return;
         static bool attr = false;
         if (!attr) {
@@ -1049,51 +1118,57 @@ static double lossT(Ctx& c, const MT* val, const MT* dval, int nprobes, const fl
         }
         const int nw = MPNN_H * 2 * MPNN_H + MPNN_H;
         const int grid = std::max(1, std::min(WG_GRID, (n + tc::WG_K - 1) / tc::WG_K));
-        launch(tc::weightGradTcKernel, grid, tc::THREADS, tc::WG_SMEM, c.s, n, (const float*)BD, X1, X2, mask, c.mpPart.p, c.status.p,
+        launch(tc::weightGradTcKernel, grid, tc::THREADS, tc::WG_SMEM, c.s, n, (const float*)BD, X1, x1Item, X2, c.mpPart.p, c.status.p,
                (int)CIPC_ST_TC_TIMEOUT);
-        launch(weightGradReduceKernel, blocksFor(nw), TB, 0, c.s, nw, MPNN_H, grid, (const float*)c.mpPart.p, gW + wOff, gW + bOff);
+        reduceWeights(nw, MPNN_H, grid, wOff, bOff);
     };
-    int nd = d.on ? c.nDynB : 0;
+    const int* none = nullptr;
+    const int nodeWarps = blocksFor(32 * nv);
+    auto edgeWarps = [](int n) { return std::max(1, (int)std::min<long long>(((long long)n * 32 + TB - 1) / TB, 148 * 32)); };
+    auto tiles = [](int n) { return std::max(1, std::min((n + LB_ITEMS - 1) / LB_ITEMS, 148 * 16)); };
     // heads
-    launch(headDiagBackKernel, blocksFor(nv), TB, 0, c.s, nv, (const float*)c.mpHeadD.p, (const int*)c.diagSlot.p, (const float*)c.mpDGS.p, wb, BD,
+    launch(headDiagBackKernel, nodeWarps, TB, 0, c.s, nv, (const float*)c.mpHeadD.p, (const int*)c.diagSlot.p, (const float*)c.mpDGS.p, wb, BD,
            DH(MPNN_L));
-    wgrad(weightGradKernel<6, MPNN_H, 0>, 6, MPNN_H, nv, (const float*)H(MPNN_L), (const float*)nullptr, (const unsigned char*)nullptr, MP_WD, MP_BD);
-    launch(headEdgeBackKernel, blocksFor(nv), TB, 0, c.s, nv, rs, re, col, (const float*)c.mpDGS.p, wb, BD, DES(MPNN_L));
-    wgrad(weightGradKernel<9, MPNN_H, MPNN_EF>, 9, MPNN_H + MPNN_EF, c.nnzb, (const float*)ES(MPNN_L), (const float*)c.mpEdgeF.p,
-          (const unsigned char*)c.mpLowS.p, MP_WO, MP_BO);
-    if (d.on) {
-        launch(headEdgeBackKernel, blocksFor(nv), TB, 0, c.s, nv, d.rs, d.re, d.col, (const float*)c.mpDGD.p, wb, BD, DED(MPNN_L));
-        wgrad(weightGradKernel<9, MPNN_H, MPNN_EF>, 9, MPNN_H + MPNN_EF, nd, (const float*)ED(MPNN_L), (const float*)c.mpEdgeFD.p,
-              (const unsigned char*)c.mpLowD.p, MP_WO, MP_BO);
+    wgrad(weightGradKernel<6, MPNN_H, 0>, 6, MPNN_H, nv, (const float*)BD, none, (const float*)H(MPNN_L), (const float*)nullptr, none, MP_WD, MP_BD);
+    if (nS) launch(headEdgeBackKernel, edgeWarps(nS), TB, 0, c.s, nS, sSlot, (const float*)c.mpDGS.p, wb, DES(MPNN_L));
+    wgrad(weightGradKernel<9, MPNN_H, MPNN_EF>, 9, MPNN_H + MPNN_EF, nS, (const float*)c.mpDGS.p, sSlot, (const float*)ES(MPNN_L),
+          (const float*)c.mpEdgeF.p, sSlot, MP_WO, MP_BO);
+    if (nE) {
+        launch(headEdgeBackKernel, edgeWarps(nE), TB, 0, c.s, nE, dSlot, (const float*)c.mpDGD.p, wb, DED(MPNN_L));
+        wgrad(weightGradKernel<9, MPNN_H, MPNN_EF>, 9, MPNN_H + MPNN_EF, nE, (const float*)c.mpDGD.p, dSlot, (const float*)ED(MPNN_L),
+              (const float*)c.mpEdgeFD.p, dSlot, MP_WO, MP_BO);
     }
     for (int l = MPNN_L - 1; l >= 0; --l) {
         const float* agg = c.mpAgg.p + (size_t)l * MPNN_H * nv;
-        launch(nodeLayerBackKernel, blocksFor(nv), TB, 0, c.s, nv, (const float*)H(l + 1), (const float*)DH(l + 1), wb + mpWh(l), BD, DH(l), c.mpDAgg.p);
-        wgradTc(nv, (const float*)H(l), agg, (const unsigned char*)nullptr, mpWh(l), mpBh(l));
-        launch(aggBackKernel, blocksFor(nv), TB, 0, c.s, nv, rs, re, col, (const float*)c.mpDAgg.p, (const int*)c.mpDeg.p, DES(l + 1));
-        if (d.on) launch(aggBackKernel, blocksFor(nv), TB, 0, c.s, nv, d.rs, d.re, d.col, (const float*)c.mpDAgg.p, (const int*)c.mpDeg.p, DED(l + 1));
-        launch(edgeLayerBackKernel, blocksFor(nv), TB, 0, c.s, nv, rs, re, col, (const float*)H(l), (const float*)ES(l + 1), (const float*)DES(l + 1),
-               wb + mpWe(l), BD, BX, DES(l), c.mpDS.p);
-        wgradTc(c.nnzb, (const float*)ES(l), (const float*)BX, (const unsigned char*)c.mpLowS.p, mpWe(l), mpBe(l));
-        if (d.on) {
-            launch(edgeLayerBackKernel, blocksFor(nv), TB, 0, c.s, nv, d.rs, d.re, d.col, (const float*)H(l), (const float*)ED(l + 1),
-                   (const float*)DED(l + 1), wb + mpWe(l), BD, BX, DED(l), c.mpDSD.p);
-            wgradTc(nd, (const float*)ED(l), (const float*)BX, (const unsigned char*)c.mpLowD.p, mpWe(l), mpBe(l));
+        launch(layerBackKernel<NodeBack>, tiles(nv), LB_THREADS, 0, c.s, nv, NodeBack{H(l + 1), DH(l + 1), DH(l), c.mpDAgg.p}, wb + mpWh(l), BD);
+        wgradTc(nv, (const float*)H(l), none, agg, mpWh(l), mpBh(l));
+        if (nS) {
+            launch(layerBackKernel<EdgeBack>, tiles(nS), LB_THREADS, 0, c.s, nS,
+                   EdgeBack{sSlot, sI, sJ, H(l), ES(l + 1), DES(l + 1), c.mpDAgg.p, c.mpDeg.p, BX, DES(l), c.mpDS.p}, wb + mpWe(l), BD);
+            wgradTc(nS, (const float*)ES(l), sSlot, (const float*)BX, mpWe(l), mpBe(l));
         }
-        launch(dsGatherKernel, blocksFor(nv), TB, 0, c.s, nv, (const int*)c.rowPtr.p, col, (const int*)c.mpMirS.p, (const float*)c.mpDS.p, d.rs, d.re,
-               d.col, (const int*)c.mpMirD.p, (const float*)c.mpDSD.p, DH(l));
+        if (nE) {
+            launch(layerBackKernel<EdgeBack>, tiles(nE), LB_THREADS, 0, c.s, nE,
+                   EdgeBack{dSlot, dI, dJ, H(l), ED(l + 1), DED(l + 1), c.mpDAgg.p, c.mpDeg.p, BX, DED(l), c.mpDSD.p}, wb + mpWe(l), BD);
+            wgradTc(nE, (const float*)ED(l), dSlot, (const float*)BX, mpWe(l), mpBe(l));
+        }
+        launch(dsGatherKernel, nodeWarps, TB, 0, c.s, nv, (const int*)c.rowPtr.p, (const int*)c.colIdx.p, (const int*)c.mpMirS.p,
+               (const int*)c.mpEdgeOfS.p, (const float*)c.mpDS.p, d.rs, d.re, d.col, (const int*)c.mpMirD.p, (const int*)c.mpEdgeOfD.p,
+               (const float*)c.mpDSD.p, DH(l));
     }
     // embeddings
-    launch(reluGradNodeKernel, blocksFor(nv * MPNN_H), TB, 0, c.s, nv, (const float*)H(0), (const float*)DH(0), BD);
-    wgrad(weightGradKernel<MPNN_H, MPNN_NF, 0>, MPNN_H, MPNN_NF, nv, (const float*)c.mpNodeF.p, (const float*)nullptr, (const unsigned char*)nullptr,
+    launch(reluGradKernel, nodeWarps, TB, 0, c.s, nv, none, (const float*)H(0), (const float*)DH(0), BD);
+    wgrad(weightGradKernel<MPNN_H, MPNN_NF, 0>, MPNN_H, MPNN_NF, nv, (const float*)BD, none, (const float*)c.mpNodeF.p, (const float*)nullptr, none,
           MP_WN0, MP_BN0);
-    launch(reluGradEdgeKernel, blocksFor(nv), TB, 0, c.s, nv, rs, re, col, (const float*)ES(0), (const float*)DES(0), BD);
-    wgrad(weightGradKernel<MPNN_H, MPNN_EF, 0>, MPNN_H, MPNN_EF, c.nnzb, (const float*)c.mpEdgeF.p, (const float*)nullptr, (const unsigned char*)c.mpLowS.p,
-          MP_WE0, MP_BE0);
-    if (d.on) {
-        launch(reluGradEdgeKernel, blocksFor(nv), TB, 0, c.s, nv, d.rs, d.re, d.col, (const float*)ED(0), (const float*)DED(0), BD);
-        wgrad(weightGradKernel<MPNN_H, MPNN_EF, 0>, MPNN_H, MPNN_EF, nd, (const float*)c.mpEdgeFD.p, (const float*)nullptr, (const unsigned char*)c.mpLowD.p,
+    if (nS) {
+        launch(reluGradKernel, edgeWarps(nS), TB, 0, c.s, nS, sSlot, (const float*)ES(0), (const float*)DES(0), BD);
+        wgrad(weightGradKernel<MPNN_H, MPNN_EF, 0>, MPNN_H, MPNN_EF, nS, (const float*)BD, none, (const float*)c.mpEdgeF.p, (const float*)nullptr, sSlot,
               MP_WE0, MP_BE0);
+    }
+    if (nE) {
+        launch(reluGradKernel, edgeWarps(nE), TB, 0, c.s, nE, dSlot, (const float*)ED(0), (const float*)DED(0), BD);
+        wgrad(weightGradKernel<MPNN_H, MPNN_EF, 0>, MPNN_H, MPNN_EF, nE, (const float*)BD, none, (const float*)c.mpEdgeFD.p, (const float*)nullptr,
+              dSlot, MP_WE0, MP_BE0);
     }
     CIPC_CUDA(cudaGetLastError());
     return loss;

@@ -63,6 +63,26 @@ def test_loss_and_gradient_match_oracle(precision):
     assert abs(l_dev - loss_o) <= LOSS_RTOL * abs(loss_o)
 
 
+@pytest.mark.parametrize("cells,copies", [(2, 1), (2, 8), (3, 9), (4, 17)])
+def test_probe_chunks_add_up(cells, copies):
+    """Probes are evaluated in chunks of 8.  k copies of one probe have its loss
+    (the mean is the same) and its gradient, but for rounding: the FP32 sum of k
+    equal terms (k - 1 times 2^-24) and the weight gradients' two-term BF16
+    split of each output gradient (2^-17 of it), so 2^-14 in norm.  Item counts
+    are off the tiles' 64 and 128 on every scene."""
+    sim = cipc.Simulator(cipc.scene_two_cubes(cells, gap=0.002), precision="mixed", precond="learned")
+    for _ in range(3):
+        sim.step()
+    sim.assemble()
+    sim.set_precond_weights(_weights())
+    probe = M.probe_vectors(sim.nv, 1, 5).astype(np.float32)
+    loss1, grad1 = sim.precond_loss(probes=probe, grad=True)
+    lossk, gradk = sim.precond_loss(probes=np.repeat(probe, copies, axis=0), grad=True)
+    assert abs(lossk - loss1) <= 1e-12 * max(1.0, abs(loss1))
+    assert np.linalg.norm(gradk - grad1) <= 2.0 ** -14 * np.linalg.norm(grad1)
+    sim.close()
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_trained_network_beats_block_jacobi(precision):
     sc = cipc.scene_cloth_drape(32, 4, newton_thr=1e-6)
