@@ -85,7 +85,7 @@ struct SimParams {
 struct DevBvh {
     int n = 0;
     DBuf<uint64_t> keys, keysAlt;
-    DBuf<int> left, right, parent, leafPrim, flags, escape;
+    DBuf<int> left, right, parent, leafPrim, flags;
     DBuf<double> lo, hi;       // 3 per node
     DBuf<double> primLo, primHi;  // 3 per primitive
     DBuf<unsigned char> sortTmp;

@@ -654,8 +654,8 @@ void cipc_gpu_destroy(cipc_gpu_context* h) {
                            &c.diagSlot, &c.hcPtr, &c.hcIdx, &c.gcPtr, &c.gcIdx, &c.selfActive, &c.selfEE, &c.eeIe, &c.ground, &c.counts, &c.runs,
                            &c.counters, &c.fricSet, &c.fricGround, &c.closeG, &c.closeS, &c.dynGKey, &c.dynGKeyAlt, &c.dynGIdx, &c.dynGIdxAlt,
                            &c.dynGStart, &c.dynGEnd, &c.dynHIdx, &c.dynHIdxAlt, &c.dynRowStart, &c.dynRowEnd, &c.dynCol, &c.dynSrcStart, &c.status,
-                           &c.faceTree.left, &c.faceTree.right, &c.faceTree.parent, &c.faceTree.leafPrim, &c.faceTree.flags, &c.faceTree.escape,
-                           &c.edgeTree.left, &c.edgeTree.right, &c.edgeTree.parent, &c.edgeTree.leafPrim, &c.edgeTree.flags, &c.edgeTree.escape, &c.mpMirS, &c.mpMirD, &c.mpDeg,
+                           &c.faceTree.left, &c.faceTree.right, &c.faceTree.parent, &c.faceTree.leafPrim, &c.faceTree.flags,
+                           &c.edgeTree.left, &c.edgeTree.right, &c.edgeTree.parent, &c.edgeTree.leafPrim, &c.edgeTree.flags, &c.mpMirS, &c.mpMirD, &c.mpDeg,
                            &c.mpRowS, &c.mpRowE};
         for (auto* d : is) d->free();
         c.mpWb.free(); c.mpEdgeOfS.free(); c.mpEdgeOfD.free(); c.pcgBar.free();
