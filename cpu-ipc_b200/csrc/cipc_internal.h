@@ -84,15 +84,14 @@ struct SimParams {
 // n-1 <= i < 2n-1 leaves in Morton order.
 struct DevBvh {
     int n = 0;
-    DBuf<uint64_t> keys, keysAlt;
-    DBuf<int> left, right, parent, leafPrim, flags;
+    const uint64_t* keys = nullptr;  // Morton keys, sorted (its part of Ctx::treeSorted)
+    DBuf<int4> links;          // internal nodes: left, right, parent, the other end of the node's leaf range
+    DBuf<int> leafParent, leafPrim, flags;
     DBuf<double> lo, hi;       // 3 per node
     DBuf<double> primLo, primHi;  // 3 per primitive
-    DBuf<unsigned char> sortTmp;
-    DBuf<double> sceneBox;     // 6
-    DBuf<double> boxPart;      // 6 per block of the scene-box reduction
+    DBuf<double> boxPart;      // 6 per block of the box kernel
     DBuf<float> rec;           // 16 per internal node: both children's boxes (rounded outward) and indices
-    DBuf<int> bigCount;        // primitives kept out of the tree (large boxes), tested by every query
+    int* bigCount = nullptr;   // primitives kept out of the tree (large boxes), tested by every query (in Ctx::treeBig)
     double bigExtent = 0;      // the box width past which a primitive is large
     // spatial-hash backend over the same primitive boxes: (cell key,
     // primitive) pairs sorted by key, and the primitives too large to insert
@@ -243,6 +242,8 @@ struct Ctx {
 
     // collision structures
     DevBvh faceTree, edgeTree;
+    DBuf<uint64_t> treeKeys, treeSorted;  // both trees' Morton keys
+    DBuf<int> treeBig;                    // their large-primitive counts
     DBuf<double> sweptPt;     // 6 per surface vertex
     DBuf<double> scratch;     // reduction scratch
     DBuf<double> sums;         // SUM_SLOTS device sums read back together
@@ -284,9 +285,6 @@ void gatherGradient(Ctx& c);           // grad = vtxGrad + element + dynamic con
 void initKappaGradE(Ctx& c, double* gE);  // inertia + tet elastic gradient into device buffer gE
 
 // ---- launchers (collision.cu) ----
-void buildBvh(Ctx& c, DevBvh& t, int n);
-void computeFaceBoxes(Ctx& c, const double* x, const double* d, double step, bool swept, const double* stepPtr = nullptr);
-void computeEdgeBoxes(Ctx& c, const double* x, const double* d, double step, bool swept, const double* stepPtr = nullptr);
 void buildCollisionSets(Ctx& c, bool rehash);
 void groundActiveSet(Ctx& c);
 bool isIntersected(Ctx& c);

@@ -54,64 +54,56 @@ __device__ __forceinline__ void sweptAdd(double lo[3], double hi[3], d3 p, d3 d,
     boxAdd(lo, hi, p - step * d);
 }
 
-__global__ void faceBoxKernel(int n, const int* faces, const double* x, const double* d, double stepVal, const double* stepPtr, int swept,
-                              double* lo, double* hi) {
-    const double step = stepPtr ? *stepPtr : stepVal;
-    CIPC_KERNEL_LOOP(f, n) {
-        double l[3], h[3];
-        boxInit(l, h);
-        for (int k = 0; k < 3; ++k) {
-            int v = faces[3 * f + k];
-            if (swept) sweptAdd(l, h, ld3(x, v), ld3(d, v), step);
-            else boxAdd(l, h, ld3(x, v));
-        }
-        for (int k = 0; k < 3; ++k) { lo[3 * f + k] = l[k]; hi[3 * f + k] = h[k]; }
-    }
-}
-__global__ void edgeBoxKernel(int n, const int* edges, const double* x, const double* d, double stepVal, const double* stepPtr, int swept,
-                              double* lo, double* hi) {
-    const double step = stepPtr ? *stepPtr : stepVal;
-    CIPC_KERNEL_LOOP(e, n) {
-        double l[3], h[3];
-        boxInit(l, h);
-        for (int k = 0; k < 2; ++k) {
-            int v = edges[2 * e + k];
-            if (swept) sweptAdd(l, h, ld3(x, v), ld3(d, v), step);
-            else boxAdd(l, h, ld3(x, v));
-        }
-        for (int k = 0; k < 3; ++k) { lo[3 * e + k] = l[k]; hi[3 * e + k] = h[k]; }
-    }
-}
+// The face and the edge tree are built by the same launches (blockIdx.y 0 and
+// 1): a build is a chain of small kernels, each a few microseconds of latency,
+// and one radix sort serves both key sets.
+struct TreeBuild {
+    int n, verts;          // primitives, vertices per primitive (3 faces, 2 edges)
+    const int* prim;       // vertex indices
+    double *plo, *phi;     // primitive boxes
+    double* part;          // 6 per block of the box kernel
+    uint64_t* keys;        // unsorted Morton keys
+    const uint64_t* sorted;
+    int* nbig;
+    int4* links;           // internal nodes: left, right, parent, the other end of the node's leaf range
+    int *leafParent, *leafPrim, *flags;
+    double *lo, *hi;
+    float* rec;
+};
+struct TreePair {
+    TreeBuild t[2];
+};
 
-// Scene box in two passes: each block reduces a strided share of the
-// primitive boxes into 6 partials, one block reduces the partials (min and
-// max do not depend on the order).  n lo/hi triples, stride 3.
-__global__ void sceneBoxKernel(int n, const double* lo, const double* hi, double* out) {
-    double l[3], h[3];
-    boxInit(l, h);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += blockDim.x * gridDim.x)
-        for (int k = 0; k < 3; ++k) { l[k] = fmin(l[k], lo[3 * i + k]); h[k] = fmax(h[k], hi[3 * i + k]); }
-    for (int k = 0; k < 3; ++k) {
-        l[k] = blockReduce(l[k], MinOp(), 1.7976931348623157e308);
-        __syncthreads();
-        h[k] = blockReduce(h[k], MaxOp(), -1.7976931348623157e308);
-        __syncthreads();
-        if (threadIdx.x == 0) { out[6 * blockIdx.x + k] = l[k]; out[6 * blockIdx.x + 3 + k] = h[k]; }
+// Primitive boxes at x, or swept from x to x - step d, and each block's box of
+// its primitives (min and max do not depend on the order).
+__global__ void primBoxKernel(TreePair pair, const double* x, const double* d, double stepVal, const double* stepPtr, int swept) {
+    const TreeBuild& t = pair.t[blockIdx.y];
+    const double step = stepPtr ? *stepPtr : stepVal;
+    double bl[3], bh[3];
+    boxInit(bl, bh);
+    CIPC_KERNEL_LOOP(f, t.n) {
+        double l[3], h[3];
+        boxInit(l, h);
+        for (int k = 0; k < t.verts; ++k) {
+            const int v = t.prim[t.verts * f + k];
+            if (swept) sweptAdd(l, h, ld3(x, v), ld3(d, v), step);
+            else boxAdd(l, h, ld3(x, v));
+        }
+        for (int k = 0; k < 3; ++k) {
+            t.plo[3 * f + k] = l[k];
+            t.phi[3 * f + k] = h[k];
+            bl[k] = fmin(bl[k], l[k]);
+            bh[k] = fmax(bh[k], h[k]);
+        }
     }
-}
-// partials (6 per block, lo then hi) of nb blocks -> box
-__global__ void sceneBoxFinalKernel(int nb, const double* part, double* out) {
-    double l[3], h[3];
-    boxInit(l, h);
-    for (int i = threadIdx.x; i < nb; i += blockDim.x)
-        for (int k = 0; k < 3; ++k) { l[k] = fmin(l[k], part[6 * i + k]); h[k] = fmax(h[k], part[6 * i + 3 + k]); }
     for (int k = 0; k < 3; ++k) {
-        l[k] = blockReduce(l[k], MinOp(), 1.7976931348623157e308);
+        bl[k] = blockReduce(bl[k], MinOp(), 1.7976931348623157e308);
         __syncthreads();
-        h[k] = blockReduce(h[k], MaxOp(), -1.7976931348623157e308);
+        bh[k] = blockReduce(bh[k], MaxOp(), -1.7976931348623157e308);
         __syncthreads();
-        if (threadIdx.x == 0) { out[k] = l[k]; out[3 + k] = h[k]; }
+        if (threadIdx.x == 0) { t.part[6 * blockIdx.x + k] = bl[k]; t.part[6 * blockIdx.x + 3 + k] = bh[k]; }
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *t.nbig = 0;
 }
 
 __device__ __forceinline__ uint32_t expandBits(uint32_t v) {
@@ -132,13 +124,33 @@ __device__ __forceinline__ uint32_t quantize(double v) {
 // tree is built over the rest, and every query tests the few large ones
 // directly - a large box would otherwise widen all its ancestors' boxes and
 // draw every query down their paths.  *nbig counts them.
-__global__ void mortonKernel(int n, const double* lo, const double* hi, const double* scene, double bigExtent, uint64_t* keys, int* nbig) {
-    CIPC_KERNEL_LOOP(i, n) {
+// Every block first reduces the box kernel's nbPart partials to the scene box.
+// The edges' keys carry bit 63: one sort puts them behind the faces'.
+__global__ void mortonKernel(TreePair pair, int nbPart, double bigExtent) {
+    const TreeBuild& t = pair.t[blockIdx.y];
+    __shared__ double scene[6];
+    {
+        double l[3], h[3];
+        boxInit(l, h);
+        for (int i = threadIdx.x; i < nbPart; i += blockDim.x)
+            for (int k = 0; k < 3; ++k) { l[k] = fmin(l[k], t.part[6 * i + k]); h[k] = fmax(h[k], t.part[6 * i + 3 + k]); }
+        for (int k = 0; k < 3; ++k) {
+            l[k] = blockReduce(l[k], MinOp(), 1.7976931348623157e308);
+            __syncthreads();
+            h[k] = blockReduce(h[k], MaxOp(), -1.7976931348623157e308);
+            __syncthreads();
+            if (threadIdx.x == 0) { scene[k] = l[k]; scene[3 + k] = h[k]; }
+        }
+        __syncthreads();
+    }
+    const uint64_t tag = (uint64_t)blockIdx.y << 63;
+    const double *lo = t.plo, *hi = t.phi;
+    CIPC_KERNEL_LOOP(i, t.n) {
         bool big = false;
         for (int k = 0; k < 3; ++k) big = big || (hi[3 * i + k] - lo[3 * i + k] > bigExtent);
         if (big) {
-            atomicAdd(nbig, 1);
-            keys[i] = (1ull << 62) | (uint32_t)i;
+            atomicAdd(t.nbig, 1);
+            t.keys[i] = tag | (1ull << 62) | (uint32_t)i;
             continue;
         }
         double c[3], q[3];
@@ -149,7 +161,7 @@ __global__ void mortonKernel(int n, const double* lo, const double* hi, const do
             q[k] = ext > 0.0 ? off / ext : 0.0;
         }
         uint32_t code = (expandBits(quantize(q[0])) << 2) | (expandBits(quantize(q[1])) << 1) | expandBits(quantize(q[2]));
-        keys[i] = ((uint64_t)code << 32) | (uint32_t)i;
+        t.keys[i] = tag | ((uint64_t)code << 32) | (uint32_t)i;
     }
 }
 
@@ -159,11 +171,20 @@ __device__ __forceinline__ int prefixLen(const uint64_t* k, int n, int a, int b)
     return x == 0 ? 64 : __clzll(x);
 }
 
-__global__ void karrasKernel(int nAll, const int* nbig, const uint64_t* keys, int* left, int* right, int* parent) {
-    const int n = nAll - *nbig;  // leaves of the tree (the large primitives stay out)
-    CIPC_KERNEL_LOOP(in, n - 1) {
-        int first, last;
-        if (in == 0) { first = 0; last = n - 1; }
+// Internal nodes (topology as CPULinearBVH::build) and the leaves' primitives.
+__global__ void karrasKernel(TreePair pair) {
+    const TreeBuild& t = pair.t[blockIdx.y];
+    const uint64_t* keys = t.sorted;
+    const int n = t.n - *t.nbig;  // leaves of the tree (the large primitives stay out)
+    CIPC_KERNEL_LOOP(in, n) {
+        t.leafPrim[in] = (int)(keys[in] & 0xffffffffu);
+        if (in == 0) {
+            if (n > 1) t.links[0].z = -1;
+            else t.leafParent[0] = -1;
+        }
+        if (in == n - 1) continue;
+        int first, last, other;
+        if (in == 0) { first = 0; last = n - 1; other = last; }
         else {
             int lp = prefixLen(keys, n, in, in - 1), rp = prefixLen(keys, n, in, in + 1);
             int dir = rp > lp ? 1 : -1;
@@ -173,7 +194,7 @@ __global__ void karrasKernel(int nAll, const int* nbig, const uint64_t* keys, in
             int len = 0;
             for (int step = maxLen >> 1; step > 0; step >>= 1)
                 if (prefixLen(keys, n, in, in + dir * (len + step)) > minp) len += step;
-            int other = in + dir * len;
+            other = in + dir * len;
             first = min(in, other); last = max(in, other);
         }
         int split;
@@ -189,25 +210,15 @@ __global__ void karrasKernel(int nAll, const int* nbig, const uint64_t* keys, in
                 if (cand < last && __clzll(fc ^ keys[cand]) > common) split = cand;
             } while (step > 1);
         }
-        int l = split, r = split + 1;
-        if (split == first) l += n - 1;
-        if (split + 1 == last) r += n - 1;
-        left[in] = l; right[in] = r;
-        parent[l] = in; parent[r] = in;
+        const bool leafL = split == first, leafR = split + 1 == last;
+        const int l = leafL ? split + n - 1 : split, r = leafR ? split + n : split + 1;
+        t.links[in].x = l;
+        t.links[in].y = r;
+        t.links[in].w = other;
+        if (leafL) t.leafParent[split] = in; else t.links[l].z = in;
+        if (leafR) t.leafParent[split + 1] = in; else t.links[r].z = in;
+        t.flags[in] = 0;
     }
-}
-
-__global__ void leafKernel(int nAll, const int* nbig, const uint64_t* keys, const double* plo, const double* phi, int* leafPrim, double* lo,
-                           double* hi, int* flags, int* parent) {
-    const int n = nAll - *nbig;
-    CIPC_KERNEL_LOOP(s, n) {
-        int prim = (int)(keys[s] & 0xffffffffu);
-        leafPrim[s] = prim;
-        int node = s + n - 1;
-        for (int k = 0; k < 3; ++k) { lo[3 * node + k] = plo[3 * prim + k]; hi[3 * node + k] = phi[3 * prim + k]; }
-        if (s < n - 1) flags[s] = 0;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) parent[0] = -1;
 }
 
 __device__ __forceinline__ int atomAddAcqRel(int* p, int v) {
@@ -216,50 +227,69 @@ __device__ __forceinline__ int atomAddAcqRel(int* p, int v) {
     return old;
 }
 
-// Bottom-up box merge: the second child to arrive at a node combines both
-// child boxes (left first, then right, as the reference's post-order merge).
-// The arrival is an acquire-release atomic: it publishes the box this thread
-// wrote for the child it came from and, for the second arrival, makes the
-// sibling's box visible.  The same thread writes the node's traversal
-// record: the boxes of both children rounded outward to FP32 (lo down, hi
-// up) and the children's node indices, 64 bytes, so that one load tests
-// both children.
-__global__ void refitKernel(int nAll, const int* nbig, const int* left, const int* right, const int* parent, double* lo, double* hi, int* flags,
-                            float* rec) {
-    const int n = nAll - *nbig;
-    if (n <= 1) return;
-    CIPC_KERNEL_LOOP(s, n) {
-        int node = s + n - 1;
-        int p = parent[node];
+// Bottom-up boxes: the second child to arrive at a node combines both child
+// boxes and goes on with the node's.  It also writes the node's traversal record:
+// the boxes of both children rounded outward to FP32 (lo down, hi up) and the
+// children's node indices, 64 bytes, so that one load tests both children.
+//
+// Bound: the chain of arrivals up the tree, each a release, an atomic and the
+// sibling's box through L2 (about 2.5 us; 42 us for 50-70k leaves).  A block owns
+// REFIT consecutive leaves, and a node whose leaf range lies among them (half the
+// levels and more) is combined through shared memory; only the rest meets in
+// global memory, by acquire-release atomics: they publish the box this thread
+// wrote for the child it came from and, for the second arrival, make the
+// sibling's box visible.
+constexpr int REFIT = 256;
+__global__ void __launch_bounds__(REFIT) refitKernel(TreePair pair) {
+    const TreeBuild& t = pair.t[blockIdx.y];
+    __shared__ double sbox[REFIT][2][6];
+    __shared__ int sflag[REFIT];
+    const int n = t.n - *t.nbig;
+    for (int base = blockIdx.x * REFIT; base < n; base += gridDim.x * REFIT) {
+        __syncthreads();  // the previous leaves' boxes are done with
+        sflag[threadIdx.x] = 0;
+        __syncthreads();
+        const int s = base + (int)threadIdx.x, top = min(base + REFIT, n);
+        if (s >= n) continue;
+        const int prim = t.leafPrim[s];
+        double b[6];
+        for (int k = 0; k < 3; ++k) { b[k] = t.plo[3 * prim + k]; b[3 + k] = t.phi[3 * prim + k]; }
+        int node = s + n - 1, p = t.leafParent[s];
+        for (int k = 0; k < 3; ++k) { t.lo[3 * (size_t)node + k] = b[k]; t.hi[3 * (size_t)node + k] = b[3 + k]; }
         for (int guard = 0; guard < 64 && p >= 0; ++guard) {
-            if (atomAddAcqRel(&flags[p], 1) == 0) break;
-            const int ch[2] = {left[p], right[p]};
-            double cb[2][6];
-            for (int q = 0; q < 2; ++q)
-                for (int k = 0; k < 3; ++k) {
-                    cb[q][k] = __ldcg(&lo[3 * ch[q] + k]);
-                    cb[q][3 + k] = __ldcg(&hi[3 * ch[q] + k]);
-                }
-            for (int k = 0; k < 3; ++k) {
-                double a = fmin(1.7976931348623157e308, cb[0][k]);
-                a = fmin(a, cb[1][k]);
-                double b = fmax(-1.7976931348623157e308, cb[0][3 + k]);
-                b = fmax(b, cb[1][3 + k]);
-                lo[3 * p + k] = a; hi[3 * p + k] = b;
+            const int4 link = t.links[p];  // left, right, parent, other end of the range
+            const int side = link.x == node ? 0 : 1;
+            double o[6];
+            if (min(p, link.w) >= base && max(p, link.w) < top) {
+                double(*slot)[6] = sbox[p - base];
+                for (int k = 0; k < 6; ++k) slot[side][k] = b[k];
+                __threadfence_block();
+                if (atomicAdd(&sflag[p - base], 1) == 0) break;
+                __threadfence_block();
+                for (int k = 0; k < 6; ++k) o[k] = reinterpret_cast<volatile double*>(slot[1 - side])[k];
+            } else {
+                if (atomAddAcqRel(&t.flags[p], 1) == 0) break;
+                const size_t sib = side == 0 ? link.y : link.x;
+                for (int k = 0; k < 3; ++k) { o[k] = __ldcg(&t.lo[3 * sib + k]); o[3 + k] = __ldcg(&t.hi[3 * sib + k]); }
             }
             float r[16];
-            for (int q = 0; q < 2; ++q)
-                for (int k = 0; k < 3; ++k) {
-                    r[6 * q + k] = __double2float_rd(cb[q][k]);
-                    r[6 * q + 3 + k] = __double2float_ru(cb[q][3 + k]);
-                }
-            r[12] = __int_as_float(ch[0]);
-            r[13] = __int_as_float(ch[1]);
+            for (int k = 0; k < 3; ++k) {
+                const double l0 = side == 0 ? b[k] : o[k], l1 = side == 0 ? o[k] : b[k];
+                const double h0 = side == 0 ? b[3 + k] : o[3 + k], h1 = side == 0 ? o[3 + k] : b[3 + k];
+                r[k] = __double2float_rd(l0); r[3 + k] = __double2float_ru(h0);
+                r[6 + k] = __double2float_rd(l1); r[9 + k] = __double2float_ru(h1);
+                b[k] = fmin(l0, l1);
+                b[3 + k] = fmax(h0, h1);
+                t.lo[3 * (size_t)p + k] = b[k];
+                t.hi[3 * (size_t)p + k] = b[3 + k];
+            }
+            r[12] = __int_as_float(link.x);
+            r[13] = __int_as_float(link.y);
             r[14] = r[15] = 0.f;
-            float4* o = reinterpret_cast<float4*>(rec) + 4 * (size_t)p;
-            for (int q = 0; q < 4; ++q) o[q] = make_float4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+            float4* out = reinterpret_cast<float4*>(t.rec) + 4 * (size_t)p;
+            for (int k = 0; k < 4; ++k) out[k] = make_float4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
             node = p;
-            p = parent[node];
+            p = link.z;
         }
     }
 }
@@ -270,7 +300,8 @@ struct BvhView {
     int nAll;         // primitives; the tree holds nAll - *nbig of them
     const int* nbig;  // primitives kept out of the tree (their keys sort last)
     const uint64_t* keys;
-    const int *left, *right, *parent, *leafPrim;
+    const int4* links;  // left, right, parent (internal nodes)
+    const int *leafParent, *leafPrim;
     const double *lo, *hi;
     const double *plo, *phi;  // primitive boxes
     const float4* rec;
@@ -287,7 +318,7 @@ int walkCap() {
     return v;
 }
 BvhView view(const DevBvh& t) {
-    return BvhView{t.bigExtent, t.n, t.bigCount.p, t.keys, t.left, t.right, t.parent, t.leafPrim, t.lo, t.hi, t.primLo, t.primHi,
+    return BvhView{t.bigExtent, t.n, t.bigCount, t.keys, t.links, t.leafParent, t.leafPrim, t.lo, t.hi, t.primLo, t.primHi,
                    reinterpret_cast<const float4*>(t.rec.p), walkCap()};
 }
 
@@ -303,10 +334,10 @@ __device__ __forceinline__ bool isLargeBox(const double* lo, const double* hi, d
 // lanes stay busy until the warp's common work is done.  The boxes of an
 // internal node's children come from its 64-byte record and are tested in FP32
 // against the query box grown by the gap and rounded outward: it contains every
-// leaf that passes the FP64 test, which alone decides what is reported.  The stack is popped from its end, which keeps it
-// near 32 times the depth; children that do not fit are walked by the lane
-// itself (walkSubtree).  f(query slot, primitive) is called by the lane that met
-// the leaf.  Sets, energy, intersection test and step bounds of the 128 x 128 cloth
+// leaf that passes the FP64 test, which alone decides what is reported.  The
+// stack is popped from its end, which keeps it near 32 times the depth; children
+// that do not fit are walked by the lane itself (walkSubtree).  f(query slot,
+// primitive) is called by the lane that met the leaf.  Sets, energy, intersection test and step bounds of the 128 x 128 cloth
 // on its cube: 5.81 -> 3.61 ms; of 27 cubes of 12 cells: 4.49 -> 3.65 ms (B200).
 constexpr int WALK_WARPS = TB / 32;
 constexpr int WALK_SLOT_SHIFT = 27;  // entries: node index in the low bits (a tree has far fewer than 2^27 nodes), query slot above
@@ -328,20 +359,20 @@ __device__ __forceinline__ bool overlapsLeaf(const BvhView& t, const WalkSmem& s
 template <class F>
 __device__ __noinline__ void walkSubtree(const BvhView& t, const WalkSmem& sm, int s, int root, int n, double gap, int* status, F& f) {
     const int firstLeaf = n - 1;
-    int cur = t.left[root];
+    int cur = t.links[root].x;
     for (int visits = 0;; ++visits) {
         if (visits > 4 * n) { raiseStatus(status, CIPC_ST_STACK_OVERFLOW); return; }
         if (overlapsLeaf(t, sm, s, cur, gap)) {
-            if (cur < firstLeaf) { cur = t.left[cur]; continue; }
+            if (cur < firstLeaf) { cur = t.links[cur].x; continue; }
             f(s, t.leafPrim[cur - firstLeaf]);
         }
-        int p = t.parent[cur];
-        while (cur != t.left[p]) {  // both of p's children are done
+        int p = cur < firstLeaf ? t.links[cur].z : t.leafParent[cur - firstLeaf];
+        while (cur != t.links[p].x) {  // both of p's children are done
             if (p == root) return;
             cur = p;
-            p = t.parent[cur];
+            p = t.links[cur].z;
         }
-        cur = t.right[p];
+        cur = t.links[p].y;
     }
 }
 
@@ -679,6 +710,54 @@ __global__ void activeEEClassKernel(const uint64_t* cand, const int* count, int 
     }
 }
 
+// The six lists of an active-set pass (candidate pairs and contacts of both
+// kinds, mollified pairs, PP/PE contacts) are sorted at once: a sort of some
+// ten thousand keys is a dozen launches of 3-9 us each, whatever it sorts.  Each
+// key is packed to the bits its indices need, below its list's number.
+struct SetLists {
+    uint64_t* key[6];  // PT candidates, PT, PP/PE, EE candidates, EE, mollified
+    int end[6];        // where the list ends in the common array
+    int faceBits, edgeBits, vertBits, tagShift;
+};
+__device__ __forceinline__ int listOf(const SetLists& s, int i) {
+    int l = 0;
+    while (i >= s.end[l]) ++l;
+    return l;
+}
+__global__ void packSetsKernel(SetLists s, uint64_t* out) {
+    CIPC_KERNEL_LOOP(i, s.end[5]) {
+        const int l = listOf(s, i);
+        const uint64_t k = s.key[l][i - (l ? s.end[l - 1] : 0)];
+        uint64_t v;
+        if (l == 2) {  // (M21 - vertex, c1, c2 + 1), the order of the fields kept
+            const uint64_t m = (1ull << s.vertBits) - 1;
+            v = ((m - (M21 - (k >> 42))) << (2 * s.vertBits)) | (((k >> 21) & M21) << s.vertBits) | (k & M21);
+        } else if (l == 5) {
+            v = ((k >> 34) << (s.edgeBits + 4)) | (k & ((1ull << 34) - 1));
+        } else {
+            v = ((k >> 32) << (l < 2 ? s.faceBits : s.edgeBits)) | (k & 0xffffffffu);
+        }
+        out[i] = ((uint64_t)l << s.tagShift) | v;
+    }
+}
+__global__ void unpackSetsKernel(SetLists s, const uint64_t* sorted) {
+    CIPC_KERNEL_LOOP(i, s.end[5]) {
+        const int l = listOf(s, i);
+        const uint64_t v = sorted[i] & ((1ull << s.tagShift) - 1);
+        uint64_t k;
+        if (l == 2) {
+            const uint64_t m = (1ull << s.vertBits) - 1;
+            k = ((M21 - (m - (v >> (2 * s.vertBits)))) << 42) | (((v >> s.vertBits) & m) << 21) | (v & m);
+        } else if (l == 5) {
+            k = ((v >> (s.edgeBits + 4)) << 34) | (v & ((1ull << (s.edgeBits + 4)) - 1));
+        } else {
+            const int b = l < 2 ? s.faceBits : s.edgeBits;
+            k = ((v >> b) << 32) | (v & ((1ull << b) - 1));
+        }
+        s.key[l][i - (l ? s.end[l - 1] : 0)] = k;
+    }
+}
+
 __global__ void decodeSelfKernel(int nPT, int nEE, int nPPE, const uint64_t* kPT, const uint64_t* kEE, const uint64_t* uniq, const int* counts,
                                  const int* surfVerts, const int* faces, const int* edges, int* out) {
     int n = nPT + nEE + nPPE;
@@ -961,15 +1040,21 @@ __global__ void groundIntersectKernel(int n, const int* ground, const double* x,
     }
 }
 
-// Stable radix sort of 64-bit keys on bits [beginBit, endBit): the bits
-// outside the range are either zero for every key or already in order.
-void sortKeys(Ctx& c, uint64_t* in, uint64_t* tmp, int n, int endBit, int beginBit = 0) {
+// Radix sort of n 64-bit keys on bits [0, endBit), in place
+void sortKeys(Ctx& c, uint64_t* keys, int n, int endBit) {
     if (n <= 1) return;
+    c.kTmp.reserve(n);
     size_t bytes = 0;
-    cub::DeviceRadixSort::SortKeys(nullptr, bytes, in, tmp, n, beginBit, endBit, c.s);
+    CIPC_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, bytes, keys, c.kTmp.p, n, 0, endBit, c.s));
     c.sortTmp.reserve(bytes + 16);
-    CIPC_CUDA(cub::DeviceRadixSort::SortKeys(c.sortTmp.p, bytes, in, tmp, n, beginBit, endBit, c.s));
-    CIPC_CUDA(cudaMemcpyAsync(in, tmp, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, c.s));
+    CIPC_CUDA(cub::DeviceRadixSort::SortKeys(c.sortTmp.p, bytes, keys, c.kTmp.p, n, 0, endBit, c.s));
+    CIPC_CUDA(cudaMemcpyAsync(keys, c.kTmp.p, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, c.s));
+}
+// CIPC_SETS_APART=1: sort the active sets' lists one by one, as for scenes of over 2^20 vertices
+bool sortSetsApart() {
+    static int v = -1;
+    if (v < 0) { const char* e = std::getenv("CIPC_SETS_APART"); v = (e && *e == '1') ? 1 : 0; }
+    return v == 1;
 }
 
 // bits needed for the values 0 .. m - 1
@@ -980,46 +1065,6 @@ int bitsFor(int m) {
 }
 
 }  // namespace
-
-// Primitive boxes of the face / edge tree at x, or swept from x to
-// x - step * d (step read from *stepPtr on the device when it is given).
-void computeFaceBoxes(Ctx& c, const double* x, const double* d, double step, bool swept, const double* stepPtr) {
-    c.faceTree.primLo.reserve(3 * std::max(1, c.nsf));
-    c.faceTree.primHi.reserve(3 * std::max(1, c.nsf));
-    if (c.nsf) launch(faceBoxKernel, blocksFor(c.nsf), TB, 0, c.s, c.nsf, c.faces, x, d, step, stepPtr, swept, c.faceTree.primLo, c.faceTree.primHi);
-}
-void computeEdgeBoxes(Ctx& c, const double* x, const double* d, double step, bool swept, const double* stepPtr) {
-    c.edgeTree.primLo.reserve(3 * std::max(1, c.nse));
-    c.edgeTree.primHi.reserve(3 * std::max(1, c.nse));
-    if (c.nse) launch(edgeBoxKernel, blocksFor(c.nse), TB, 0, c.s, c.nse, c.edges, x, d, step, stepPtr, swept, c.edgeTree.primLo, c.edgeTree.primHi);
-}
-
-void buildBvh(Ctx& c, DevBvh& t, int n) {
-    t.n = n;
-    if (n <= 0) return;
-    int nn = 2 * n - 1;
-    t.keys.reserve(n); t.keysAlt.reserve(n);
-    t.left.reserve(nn); t.right.reserve(nn); t.parent.reserve(nn); t.leafPrim.reserve(n); t.flags.reserve(n);
-    t.lo.reserve(3 * nn); t.hi.reserve(3 * nn); t.sceneBox.reserve(6);
-    const int nbBox = std::max(1, std::min(148, (n + 255) / 256));
-    t.boxPart.reserve(6 * (size_t)nbBox);
-    launch(sceneBoxKernel, nbBox, 256, 0, c.s, n, t.primLo, t.primHi, t.boxPart);
-    launch(sceneBoxFinalKernel, 1, 256, 0, c.s, nbBox, (const double*)t.boxPart, t.sceneBox);
-    t.bigCount.reserve(1);
-    CIPC_CUDA(cudaMemsetAsync(t.bigCount.p, 0, sizeof(int), c.s));
-    const double bigExtent = t.bigExtent = 0.1 * std::sqrt(c.P.bboxDiag2);
-    launch(mortonKernel, blocksFor(n), TB, 0, c.s, n, t.primLo, t.primHi, t.sceneBox, bigExtent, t.keys, t.bigCount.p);
-    // keys are (code << 32) | index (bit 62: kept out of the tree), written in
-    // index order: a stable sort on bits 32-62 gives the order of a sort on
-    // the whole key
-    sortKeys(c, t.keys, t.keysAlt, n, 63, 32);
-    const int* nbig = t.bigCount.p;
-    if (n > 1) launch(karrasKernel, blocksFor(n - 1), TB, 0, c.s, n, nbig, t.keys, t.left, t.right, t.parent);
-    launch(leafKernel, blocksFor(n), TB, 0, c.s, n, nbig, t.keys, t.primLo, t.primHi, t.leafPrim, t.lo, t.hi, t.flags, t.parent);
-    t.rec.reserve(16 * (size_t)std::max(1, n - 1));
-    if (n > 1) launch(refitKernel, blocksFor(n), TB, 0, c.s, n, nbig, t.left, t.right, t.parent, t.lo, t.hi, t.flags, t.rec.p);
-    CIPC_CUDA(cudaGetLastError());
-}
 
 // The spatial-hash tables of one primitive set from its boxes (primLo/Hi).
 void buildHash(Ctx& c, DevBvh& t, int n) {
@@ -1068,10 +1113,55 @@ HashView hview(Ctx& c, const DevBvh& t) {
                     t.primLo, t.primHi};
 }
 
-// The broad-phase structure of one primitive set, LBVH or spatial hash.
-void buildBroad(Ctx& c, DevBvh& t, int n) {
-    if (c.broadPhase == CIPC_BROAD_PHASE_SPATIAL_HASH) buildHash(c, t, n);
-    else buildBvh(c, t, n);
+// Both trees over the primitive boxes at x, or swept from x to x - step * d
+// (step read from *stepPtr on the device when it is given).
+static void buildTrees(Ctx& c, const double* x, const double* d, double step, bool swept, const double* stepPtr) {
+    TreePair pair{};
+    const int total = c.nsf + c.nse;
+    c.treeKeys.reserve(std::max(1, total));
+    c.treeSorted.reserve(std::max(1, total));
+    c.treeBig.reserve(2);
+    // one share of the boxes per block; the same count for both trees, whose
+    // Morton kernel reduces the partials
+    const int nbBox = std::max(1, std::min(148, (std::max(c.nsf, c.nse) + 255) / 256));
+    const bool hash = c.broadPhase == CIPC_BROAD_PHASE_SPATIAL_HASH;
+    for (int k = 0; k < 2; ++k) {
+        DevBvh& t = k == 0 ? c.faceTree : c.edgeTree;
+        const int n = k == 0 ? c.nsf : c.nse, nn = std::max(1, 2 * n - 1);
+        t.n = n;
+        t.bigExtent = 0.1 * std::sqrt(c.P.bboxDiag2);
+        t.primLo.reserve(3 * (size_t)std::max(1, n)); t.primHi.reserve(3 * (size_t)std::max(1, n));
+        t.boxPart.reserve(6 * (size_t)nbBox);
+        if (!hash) {
+            t.links.reserve(std::max(1, n)); t.leafParent.reserve(std::max(1, n)); t.leafPrim.reserve(std::max(1, n)); t.flags.reserve(std::max(1, n));
+            t.lo.reserve(3 * (size_t)nn); t.hi.reserve(3 * (size_t)nn);
+            t.rec.reserve(16 * (size_t)std::max(1, n - 1));
+        }
+        t.keys = c.treeSorted.p + (k == 0 ? 0 : c.nsf);
+        t.bigCount = c.treeBig.p + k;
+        pair.t[k] = TreeBuild{n, k == 0 ? 3 : 2, k == 0 ? c.faces.p : c.edges.p, t.primLo, t.primHi, t.boxPart, c.treeKeys.p + (k == 0 ? 0 : c.nsf),
+                              t.keys, t.bigCount, t.links, t.leafParent, t.leafPrim, t.flags, t.lo, t.hi, t.rec};
+    }
+    launch(primBoxKernel, dim3(nbBox, 2), 256, 0, c.s, pair, x, d, step, stepPtr, swept ? 1 : 0);
+    if (hash) {
+        buildHash(c, c.faceTree, c.nsf);
+        buildHash(c, c.edgeTree, c.nse);
+        return;
+    }
+    const int most = std::max(1, std::max(c.nsf, c.nse));
+    launch(mortonKernel, dim3(std::min(blocksFor(most), 148 * 2), 2), TB, 0, c.s, pair, nbBox, c.faceTree.bigExtent);
+    // keys are (tree << 63 | code << 32) | index (bit 62: kept out of the tree),
+    // written in index order: a stable sort on bits 32-63 gives the order of a
+    // sort on the whole key
+    if (total > 0) {
+        size_t bytes = 0;
+        CIPC_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, bytes, c.treeKeys.p, c.treeSorted.p, total, 32, 64, c.s));
+        c.sortTmp.reserve(bytes + 16);
+        CIPC_CUDA(cub::DeviceRadixSort::SortKeys(c.sortTmp.p, bytes, c.treeKeys.p, c.treeSorted.p, total, 32, 64, c.s));
+    }
+    launch(karrasKernel, dim3(blocksFor(most), 2), TB, 0, c.s, pair);
+    launch(refitKernel, dim3(std::max(1, std::min((most + REFIT - 1) / REFIT, 148 * 8)), 2), REFIT, 0, c.s, pair);
+    CIPC_CUDA(cudaGetLastError());
 }
 
 // Calls k(view) with the selected backend's view of tree t.
@@ -1081,12 +1171,7 @@ void withView(Ctx& c, const DevBvh& t, K k) {
     else k(view(t));
 }
 
-static void buildStaticTrees(Ctx& c) {
-    computeFaceBoxes(c, c.x, c.x, 0.0, false);
-    buildBroad(c, c.faceTree, c.nsf);
-    computeEdgeBoxes(c, c.x, c.x, 0.0, false);
-    buildBroad(c, c.edgeTree, c.nse);
-}
+static void buildStaticTrees(Ctx& c) { buildTrees(c, c.x, c.x, 0.0, false, nullptr); }
 
 // Ground::calculateActivateSet: the surface vertices within dHat of the
 // ground, in order, into c.ground; their count lands in counters[15] (read
@@ -1165,16 +1250,35 @@ void buildCollisionSets(Ctx& c, bool rehash) {
         // last launch could write
         if (!fits) throw std::runtime_error("active-set candidate counts exceed their buffers after four attempts");
         c.nCcdPT = cnt[0]; c.nPT = cnt[1]; c.nPPERaw = cnt[2]; c.nCcdEE = cnt[3]; c.nEE = cnt[4]; c.nMoll = cnt[5];
-        int mx = std::max(std::max(std::max(cnt[0], cnt[1]), std::max(cnt[2], cnt[3])), std::max(cnt[4], cnt[5]));
-        c.kTmp.reserve(std::max(mx, 1));
-        // pair keys (query << 32 | primitive), mollified (eI << 34 | eJ << 4 | type)
-        const int ptBits = 32 + bitsFor(c.nsv), eeBits = 32 + bitsFor(c.nse), mollBits = std::min(64, 34 + bitsFor(c.nse));
-        sortKeys(c, c.ccdPT, c.kTmp, cnt[0], ptBits);
-        sortKeys(c, c.kPT, c.kTmp, cnt[1], ptBits);
-        sortKeys(c, c.kPPE, c.kTmp, cnt[2], 63);
-        sortKeys(c, c.ccdEE, c.kTmp, cnt[3], eeBits);
-        sortKeys(c, c.kEE, c.kTmp, cnt[4], eeBits);
-        sortKeys(c, c.kMoll, c.kTmp, cnt[5], mollBits);
+        {
+            SetLists lists{};
+            uint64_t* keys[6] = {c.ccdPT.p, c.kPT.p, c.kPPE.p, c.ccdEE.p, c.kEE.p, c.kMoll.p};
+            long long n = 0;
+            for (int k = 0; k < 6; ++k) {
+                lists.key[k] = keys[k];
+                n += cnt[k];
+                if (n > 0x7fffffff) throw std::runtime_error("the active-set candidates exceed 2^31");
+                lists.end[k] = (int)n;
+            }
+            // PP/PE fields hold up to nv (c2 + 1); edge pairs of the mollified list 4 type bits
+            lists.faceBits = bitsFor(c.nsf); lists.edgeBits = bitsFor(c.nse); lists.vertBits = bitsFor(c.nv + 1);
+            lists.tagShift = std::max(std::max(bitsFor(c.nsv) + lists.faceBits, 2 * lists.edgeBits + 4), 3 * lists.vertBits);
+            if (lists.tagShift > 61 || sortSetsApart()) {
+                // over 2^20 vertices: three vertex fields and the list's number do not fit 64 bits
+                const int endBit[6] = {32 + bitsFor(c.nsv), 32 + bitsFor(c.nsv), 63, 32 + bitsFor(c.nse), 32 + bitsFor(c.nse),
+                                       std::min(64, 34 + bitsFor(c.nse))};
+                for (int k = 0; k < 6; ++k) sortKeys(c, keys[k], cnt[k], endBit[k]);
+            } else if (n > 1) {
+                c.kTmp.reserve(2 * (size_t)n);
+                uint64_t *in = c.kTmp.p, *out = c.kTmp.p + n;
+                launch(packSetsKernel, blocksFor((int)n), TB, 0, c.s, lists, in);
+                size_t bytes = 0;
+                CIPC_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, bytes, in, out, (int)n, 0, lists.tagShift + 3, c.s));
+                c.sortTmp.reserve(bytes + 16);
+                CIPC_CUDA(cub::DeviceRadixSort::SortKeys(c.sortTmp.p, bytes, in, out, (int)n, 0, lists.tagShift + 3, c.s));
+                launch(unpackSetsKernel, blocksFor((int)n), TB, 0, c.s, lists, (const uint64_t*)out);
+            }
+        }
         // merge PP/PE duplicates (multiplicity)
         int nu = 0;
         c.uniq.reserve(std::max(cnt[2], 1));
@@ -1322,10 +1426,7 @@ static void fullPTDevice(Ctx& c, const double* d, double stepVal, const double* 
 // Swept build with the entry step, then Self_largestFeasibleStepSize_CCD.
 double fullCCDDir(Ctx& c, const double* d, double alpha) {
     double step = alpha;
-    computeFaceBoxes(c, c.x, d, step, true);
-    buildBroad(c, c.faceTree, c.nsf);
-    computeEdgeBoxes(c, c.x, d, step, true);
-    buildBroad(c, c.edgeTree, c.nse);
+    buildTrees(c, c.x, d, step, true, nullptr);
     c.stepScal.reserve(16);
     double* sm = c.stepScal.p + 12;  // [12] minimum, [13] pair count
     // one pass (point-triangle or edge-edge) with the host's entry step; a
@@ -1414,10 +1515,7 @@ double stepBoundsDevice(Ctx& c) {
             launch(surfMoveKernel, blocksFor(c.nsv), TB, 0, c.s, c.nsv, c.surfVerts, c.dir, c.energyBuf);
             deviceMaxTo(c, c.energyBuf, c.nsv, s + 2);
         }
-        computeFaceBoxes(c, c.x, c.dir, 0.0, true, s + 3);
-        buildBroad(c, c.faceTree, c.nsf);
-        computeEdgeBoxes(c, c.x, c.dir, 0.0, true, s + 3);
-        buildBroad(c, c.edgeTree, c.nse);
+        buildTrees(c, c.x, c.dir, 0.0, true, s + 3);
         ccdPairsReserve(c);
         CIPC_CUDA(cudaMemsetAsync(c.ccdPairCount.p, 0, 2 * sizeof(int), c.s));
         if (c.nsv) {

@@ -94,6 +94,7 @@ struct DynOut {
     uint64_t* hKey;
     void* hVal;
     int mixed;
+    int colBits;  // block keys are row << colBits | column, the bits a vertex needs: the sort runs over twice as many
 };
 
 __device__ __forceinline__ void putH(const DynOut& o, size_t e, int k, double v) {
@@ -111,7 +112,7 @@ __device__ void writeBlocks(const DynOut& o, size_t hBase, const double* A, int 
         int a = blk / 4, b = blk % 4;
         size_t slot = hBase + blk;
         bool valid = a < np && b < np && btype[idx[a]] == 0 && btype[idx[b]] == 0;
-        if (k == 0) o.hKey[slot] = valid ? (((uint64_t)(uint32_t)idx[a] << 32) | (uint32_t)idx[b]) : HSENT;
+        if (k == 0) o.hKey[slot] = valid ? (((uint64_t)(uint32_t)idx[a] << o.colBits) | (uint32_t)idx[b]) : HSENT;
         double v = valid ? A[(3 * a + k / 3) * ld + 3 * b + k % 3] : 0.0;
         putH(o, slot, k, v);
     }
@@ -442,7 +443,7 @@ __global__ void frictionSelfKernel(int n, const int* fset, const double* x, cons
             int a = blk / 4, b = blk % 4;
             size_t slot = hBase + 16 * (size_t)i + blk;
             bool valid = a < np && b < np && btype[idx[a]] == 0 && btype[idx[b]] == 0;
-            o.hKey[slot] = valid ? (((uint64_t)(uint32_t)idx[a] << 32) | (uint32_t)idx[b]) : HSENT;
+            o.hKey[slot] = valid ? (((uint64_t)(uint32_t)idx[a] << o.colBits) | (uint32_t)idx[b]) : HSENT;
             for (int r = 0; r < 3; ++r)
                 for (int q = 0; q < 3; ++q) {
                     double v = 0;
@@ -560,34 +561,30 @@ __global__ void gradSegKernel(int n, const int* keys, int* start, int* end) {
         if (i == n - 1 || keys[i + 1] != k) end[k] = i + 1;
     }
 }
-__global__ void headFlagKernel(int n, const uint64_t* keys, int* flags) {
+// segment heads of the sorted keys, and the number of keys before the
+// sentinels (which sort last)
+__global__ void headFlagKernel(int n, const uint64_t* keys, int* flags, int* nValid) {
     CIPC_KERNEL_LOOP(i, n) {
-        uint64_t k = keys[i];
-        flags[i] = (k != HSENT && (i == 0 || keys[i - 1] != k)) ? 1 : 0;
+        const uint64_t k = keys[i];
+        const bool valid = k != HSENT;
+        flags[i] = (valid && (i == 0 || keys[i - 1] != k)) ? 1 : 0;
+        if (valid ? i == n - 1 || keys[i + 1] == HSENT : i == 0) *nValid = valid ? i + 1 : 0;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) flags[n] = 0;  // so that the scan's last entry is the count of heads
 }
-__global__ void uniqueKernel(int n, const uint64_t* keys, const int* flags, const int* pos, int* col, int* srcStart) {
+__global__ void uniqueKernel(int n, const uint64_t* keys, const int* flags, const int* pos, int colBits, int* col, int* srcStart) {
     CIPC_KERNEL_LOOP(i, n) {
         if (!flags[i]) continue;
         int u = pos[i];
-        col[u] = (int)(keys[i] & 0xffffffffu);
+        col[u] = (int)(keys[i] & ((1ull << colBits) - 1));
         srcStart[u] = i;
     }
 }
-// Number of non-sentinel entries in a sorted key array (sentinels sort last).
-__global__ void validCountKernel(int n, const uint64_t* keys, int* out) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        int mid = (lo + hi) >> 1;
-        if (keys[mid] == HSENT) hi = mid; else lo = mid + 1;
-    }
-    *out = lo;
-}
-__global__ void rowBoundsKernel(int nu, const int* srcStart, const uint64_t* keys, int* rowStart, int* rowEnd) {
+__global__ void rowBoundsKernel(int nu, const int* srcStart, const uint64_t* keys, int colBits, int* rowStart, int* rowEnd) {
     CIPC_KERNEL_LOOP(u, nu) {
-        int r = (int)(keys[srcStart[u]] >> 32);
-        int rPrev = u > 0 ? (int)(keys[srcStart[u - 1]] >> 32) : -1;
-        int rNext = u + 1 < nu ? (int)(keys[srcStart[u + 1]] >> 32) : -1;
+        int r = (int)(keys[srcStart[u]] >> colBits);
+        int rPrev = u > 0 ? (int)(keys[srcStart[u - 1]] >> colBits) : -1;
+        int rNext = u + 1 < nu ? (int)(keys[srcStart[u + 1]] >> colBits) : -1;
         if (r != rPrev) rowStart[r] = u;
         if (r != rNext) rowEnd[r] = u + 1;
     }
@@ -609,11 +606,19 @@ __global__ void iotaKernel(int n, int* a) { CIPC_KERNEL_LOOP(i, n) a[i] = i; }
 
 }  // namespace
 
+// bits of a vertex index, the sentinels (all ones) apart: 2^bits > nv
+static int vertexBits(const Ctx& c) {
+    int b = 1;
+    while (b < 31 && (1ll << b) <= c.nv) ++b;
+    return b;
+}
+
 static DynOut dynOut(Ctx& c) {
     DynOut o;
     o.gKey = c.dynGKey; o.gVal = c.dynGVal; o.hKey = c.dynHKey;
     o.hVal = c.mixed ? (void*)c.dynHValF.p : (void*)c.dynHValD.p;
     o.mixed = c.mixed;
+    o.colBits = vertexBits(c);
     return o;
 }
 
@@ -665,6 +670,7 @@ int contactAssemble(Ctx& c) {
 
 void finalizeDynamic(Ctx& c) {
     int ng = c.nDynG, nh = c.nDynH;
+    const int bits = vertexBits(c);
     c.dynGStart.reserve(c.nv); c.dynGEnd.reserve(c.nv);
     CIPC_CUDA(cudaMemsetAsync(c.dynGStart.p, 0, sizeof(int) * c.nv, c.s));
     CIPC_CUDA(cudaMemsetAsync(c.dynGEnd.p, 0, sizeof(int) * c.nv, c.s));
@@ -675,39 +681,34 @@ void finalizeDynamic(Ctx& c) {
     if (ng > 0) {
         launch(iotaKernel, blocksFor(ng), TB, 0, c.s, ng, c.dynGIdxAlt);
         size_t bytes = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, bytes, c.dynGKey.p, c.dynGKeyAlt.p, c.dynGIdxAlt.p, c.dynGIdx.p, ng, 0, 32, c.s);
+        cub::DeviceRadixSort::SortPairs(nullptr, bytes, c.dynGKey.p, c.dynGKeyAlt.p, c.dynGIdxAlt.p, c.dynGIdx.p, ng, 0, bits, c.s);
         c.sortTmp.reserve(bytes + 16);
-        CIPC_CUDA(cub::DeviceRadixSort::SortPairs(c.sortTmp.p, bytes, c.dynGKey.p, c.dynGKeyAlt.p, c.dynGIdxAlt.p, c.dynGIdx.p, ng, 0, 32, c.s));
+        CIPC_CUDA(cub::DeviceRadixSort::SortPairs(c.sortTmp.p, bytes, c.dynGKey.p, c.dynGKeyAlt.p, c.dynGIdxAlt.p, c.dynGIdx.p, ng, 0, bits, c.s));
         launch(gradSegKernel, blocksFor(ng), TB, 0, c.s, ng, c.dynGKeyAlt, c.dynGStart, c.dynGEnd);
     }
     if (nh > 0) {
         launch(iotaKernel, blocksFor(nh), TB, 0, c.s, nh, c.dynHIdxAlt);
         size_t bytes = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, bytes, c.dynHKey.p, c.dynHKeyAlt.p, c.dynHIdxAlt.p, c.dynHIdx.p, nh, 0, 64, c.s);
+        cub::DeviceRadixSort::SortPairs(nullptr, bytes, c.dynHKey.p, c.dynHKeyAlt.p, c.dynHIdxAlt.p, c.dynHIdx.p, nh, 0, 2 * bits, c.s);
         c.sortTmp.reserve(bytes + 16);
-        CIPC_CUDA(cub::DeviceRadixSort::SortPairs(c.sortTmp.p, bytes, c.dynHKey.p, c.dynHKeyAlt.p, c.dynHIdxAlt.p, c.dynHIdx.p, nh, 0, 64, c.s));
+        CIPC_CUDA(cub::DeviceRadixSort::SortPairs(c.sortTmp.p, bytes, c.dynHKey.p, c.dynHKeyAlt.p, c.dynHIdxAlt.p, c.dynHIdx.p, nh, 0, 2 * bits, c.s));
         c.counts.reserve(nh + 1);
         c.runs.reserve(nh + 1);
-        launch(headFlagKernel, blocksFor(nh), TB, 0, c.s, nh, c.dynHKeyAlt, c.counts);
+        c.counters.reserve(16);
+        launch(headFlagKernel, blocksFor(nh), TB, 0, c.s, nh, c.dynHKeyAlt, c.counts, c.counters.p + 9);
         size_t b2 = 0;
         cub::DeviceScan::ExclusiveSum(nullptr, b2, c.counts.p, c.runs.p, nh + 1, c.s);
         c.sortTmp.reserve(b2 + 16);
-        // flags[nh] must be 0 so that runs[nh] is the unique count
-        CIPC_CUDA(cudaMemsetAsync(c.counts.p + nh, 0, sizeof(int), c.s));
         CIPC_CUDA(cub::DeviceScan::ExclusiveSum(c.sortTmp.p, b2, c.counts.p, c.runs.p, nh + 1, c.s));
-        int nu = 0;
+        int nu = 0, nValid = 0;
         CIPC_CUDA(cudaMemcpyAsync(&nu, c.runs.p + nh, sizeof(int), cudaMemcpyDeviceToHost, c.s));
+        CIPC_CUDA(cudaMemcpyAsync(&nValid, c.counters.p + 9, sizeof(int), cudaMemcpyDeviceToHost, c.s));
         hostSync(c);
         c.nDynB = nu;
         if (nu > 0) {
             c.dynCol.reserve(nu); c.dynSrcStart.reserve(nu);
-            launch(uniqueKernel, blocksFor(nh), TB, 0, c.s, nh, c.dynHKeyAlt, c.counts, c.runs, c.dynCol, c.dynSrcStart);
-            launch(rowBoundsKernel, blocksFor(nu), TB, 0, c.s, nu, c.dynSrcStart, c.dynHKeyAlt, c.dynRowStart, c.dynRowEnd);
-            c.counters.reserve(16);
-            launch(validCountKernel, 1, 1, 0, c.s, nh, c.dynHKeyAlt, c.counters.p + 9);
-            int nValid = 0;
-            CIPC_CUDA(cudaMemcpyAsync(&nValid, c.counters.p + 9, sizeof(int), cudaMemcpyDeviceToHost, c.s));
-            hostSync(c);
+            launch(uniqueKernel, blocksFor(nh), TB, 0, c.s, nh, c.dynHKeyAlt, c.counts, c.runs, bits, c.dynCol, c.dynSrcStart);
+            launch(rowBoundsKernel, blocksFor(nu), TB, 0, c.s, nu, c.dynSrcStart, c.dynHKeyAlt, bits, c.dynRowStart, c.dynRowEnd);
             if (c.mixed) {
                 c.dynBF.reserve((size_t)9 * nu);
                 launch(dynReduceKernel<float>, blocksFor(nu), TB, 0, c.s, nu, nValid, c.dynSrcStart, c.dynHIdx, c.dynHValF, c.dynBF);

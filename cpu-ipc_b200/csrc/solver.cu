@@ -642,8 +642,8 @@ void cipc_gpu_destroy(cipc_gpu_context* h) {
                               &c.fricLambda, &c.fricCoord, &c.fricBasis, &c.fricGLambda, &c.closeGVal, &c.closeSVal, &c.dynGVal, &c.dynHValD,
                               &c.dynBD, &c.rhs, &c.sol, &c.r, &c.z, &c.p, &c.Ap, &c.Dinv, &c.red, &c.corrX, &c.corrR, &c.sweptPt, &c.scratch,
                               &c.scal, &c.energyBuf, &c.sums, &c.mpS, &c.mpT, &c.pcgPipe, &c.pcgParts,
-                              &c.faceTree.lo, &c.faceTree.hi, &c.faceTree.primLo, &c.faceTree.primHi, &c.faceTree.sceneBox, &c.edgeTree.lo,
-                              &c.edgeTree.hi, &c.edgeTree.primLo, &c.edgeTree.primHi, &c.edgeTree.sceneBox, &c.faceTree.boxPart, &c.edgeTree.boxPart};
+                              &c.faceTree.lo, &c.faceTree.hi, &c.faceTree.primLo, &c.faceTree.primHi, &c.edgeTree.lo,
+                              &c.edgeTree.hi, &c.edgeTree.primLo, &c.edgeTree.primHi, &c.faceTree.boxPart, &c.edgeTree.boxPart};
         for (auto* d : ds) d->free();
         DBuf<float>* fs[] = {&c.valF, &c.elemHF, &c.dynHValF, &c.dynBF, &c.rF, &c.zF, &c.pF, &c.ApF, &c.xF, &c.DinvF, &c.mpW, &c.mpG, &c.mpM, &c.mpV,
                              &c.mpNodeF, &c.mpEdgeF, &c.mpEdgeFD, &c.mpH, &c.mpAgg, &c.mpES, &c.mpED, &c.mpHeadD, &c.mpGS, &c.mpGD,
@@ -654,19 +654,19 @@ void cipc_gpu_destroy(cipc_gpu_context* h) {
                            &c.diagSlot, &c.hcPtr, &c.hcIdx, &c.gcPtr, &c.gcIdx, &c.selfActive, &c.selfEE, &c.eeIe, &c.ground, &c.counts, &c.runs,
                            &c.counters, &c.fricSet, &c.fricGround, &c.closeG, &c.closeS, &c.dynGKey, &c.dynGKeyAlt, &c.dynGIdx, &c.dynGIdxAlt,
                            &c.dynGStart, &c.dynGEnd, &c.dynHIdx, &c.dynHIdxAlt, &c.dynRowStart, &c.dynRowEnd, &c.dynCol, &c.dynSrcStart, &c.status,
-                           &c.faceTree.left, &c.faceTree.right, &c.faceTree.parent, &c.faceTree.leafPrim, &c.faceTree.flags,
-                           &c.edgeTree.left, &c.edgeTree.right, &c.edgeTree.parent, &c.edgeTree.leafPrim, &c.edgeTree.flags, &c.mpMirS, &c.mpMirD, &c.mpDeg,
+                           &c.faceTree.leafParent, &c.faceTree.leafPrim, &c.faceTree.flags, &c.edgeTree.leafParent, &c.edgeTree.leafPrim,
+                           &c.edgeTree.flags, &c.treeBig, &c.mpMirS, &c.mpMirD, &c.mpDeg,
                            &c.mpRowS, &c.mpRowE};
         for (auto* d : is) d->free();
         c.mpWb.free(); c.mpEdgeOfS.free(); c.mpEdgeOfD.free(); c.pcgBar.free();
         DBuf<uint64_t>* us[] = {&c.ccdPT, &c.ccdEE, &c.kPT, &c.kEE, &c.kMoll, &c.kPPE, &c.kTmp, &c.uniq, &c.dynHKey, &c.dynHKeyAlt,
-                                &c.faceTree.keys, &c.faceTree.keysAlt, &c.edgeTree.keys, &c.edgeTree.keysAlt};
+                                &c.treeKeys, &c.treeSorted};
         for (auto* d : us) d->free();
-        c.sortTmp.free(); c.groundTmp.free(); c.barrierUpper.free(); c.ccdPairs.free(); c.ccdPairCount.free(); c.stepScal.free(); c.faceTree.sortTmp.free(); c.edgeTree.sortTmp.free();
+        c.sortTmp.free(); c.groundTmp.free(); c.barrierUpper.free(); c.ccdPairs.free(); c.ccdPairCount.free(); c.stepScal.free(); c.faceTree.links.free(); c.edgeTree.links.free();
         c.gLptr.free(); c.gLcol.free(); c.gLslot.free(); c.gUptr.free(); c.gUcol.free(); c.gUslot.free(); c.gLval.free(); c.gUval.free();
         for (DevBvh* t : {&c.faceTree, &c.edgeTree}) {
             t->hashKey.free(); t->hashKeyAlt.free(); t->hashPrim.free(); t->hashPrimAlt.free(); t->hashCount.free(); t->hashOffset.free();
-            t->hashBig.free(); t->hashBigFlag.free(); t->hashTmp.free(); t->bigCount.free();
+            t->hashBig.free(); t->hashBigFlag.free(); t->hashTmp.free();
         }
         for (cudaEvent_t e : c.profEv) cudaEventDestroy(e);
         if (c.s) cudaStreamDestroy(c.s);
