@@ -101,6 +101,16 @@ struct DevBvh {
     DBuf<unsigned char> hashTmp;
 };
 
+// A static block pattern in tiles of 8 rows for the streaming PCG: the rows'
+// source slots (ptr, slot; empty for the matrix itself), the tiles' step
+// offsets, and per step 32 columns and 32 blocks.
+struct SellRows {
+    DBuf<int> ptr, slot, tile, col;
+    DBuf<unsigned char> val;
+    int steps = 0;
+    void free() { ptr.free(); slot.free(); tile.free(); col.free(); val.free(); }
+};
+
 struct Ctx {
     // sizes
     int nv = 0, nt = 0, nf = 0, nb = 0, nsf = 0, nsv = 0, nse = 0;
@@ -205,14 +215,8 @@ struct Ctx {
     int lastPcgLaunchIters = 0;
     DBuf<unsigned> pcgBar;              // grid-barrier counters of the persistent PCG
     DBuf<double> pcgPipe, pcgParts;     // pipelined PCG: six recurrence vectors, two sets of partial sums
-    // the factor packed for the streaming PCG: lower part (columns <= row) and
-    // transposed part (columns >= row, diagonal transposed) of the static
-    // slots as compact rows of FP16 blocks (9 halves each); the index lists
-    // depend only on the static pattern and are built once
-    DBuf<int> gLptr, gLcol, gLslot, gUptr, gUcol, gUslot;
-    DBuf<uint16_t> gLval, gUval;
-    int nGL = 0, nGU = 0;
-    bool factorPacked = false;
+    DBuf<double> pcgGather, pcgState;   // streaming PCG: four gathered vectors, 4 entries per row; the recurrence vectors
+    SellRows sellA, sellL, sellU;       // streaming PCG: the static matrix, G and G^T in tiles
     int pcgSliceMax = -1;               // cached pipelined PCG: largest static-slot count of a block's rows
     int pcgSliceRows = 0;               // the block row count pcgSliceMax was computed for
     bool assembled = false;             // a Newton system has been assembled

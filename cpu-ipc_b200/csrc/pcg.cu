@@ -273,6 +273,15 @@ __global__ void accumulateKernel(int n3, const float* d, double* x) {
 // results are reproducible.  The barrier spin is bounded: on timeout it sets
 // an error flag and the kernel returns.
 // ---------------------------------------------------------------------------
+// A matrix in tiles of 8 rows (streaming variant, below): tile t holds steps
+// [tile[t], tile[t + 1]); a step holds one 3x3 block for each of a warp's 32
+// lanes, its column (-1: none) and its nine values.
+struct SellView {
+    const int* tile;
+    const int* col;
+    const void* val;
+};
+
 template <class MT, class VT>
 struct PcgArgs {
     int nv;
@@ -285,14 +294,16 @@ struct PcgArgs {
     // learned factor (null for block-Jacobi): S 9 per vertex, G slot-aligned
     const double* S;
     const float *gS, *gD;
-    // the static part of G packed by rows (null: read gS): lower part and
-    // transposed part, FP16 blocks with their columns and row offsets
-    const __half *gL, *gU;
-    const int *gLptr, *gLcol, *gUptr, *gUcol;
     VT* t;
     const VT* b;
     VT *x, *r, *z, *p, *Ap;
-    VT *u, *w, *mA, *mB, *q, *s;  // pipelined variant only
+    VT *u, *w, *mA, *mB, *q, *s;  // pipelined variants only
+    // streaming variant: gathered vectors padded to 4 entries per row, the
+    // tiled matrix and factor parts, the tiles a block owns at most, whether
+    // the recurrence vectors live in shared memory, and else where they live
+    VT *g0, *g1, *g2, *g3, *state;
+    SellView sA, sL, sU;
+    int resident, tilesPerBlock;
     double *partA, *partB, *partC;
     double* pp;                   // pipelined variant: two sets of three partial arrays, PIPE_PMAX each
     int sliceMax;                 // cached variant: static slots of the largest block row range
@@ -487,24 +498,7 @@ __device__ __forceinline__ void rowSpmv(const PcgArgs<MT, VT>& a, int row, int l
 // (G^T u)_row (TR = true: mirror slots and the transposed diagonal block)
 template <bool TR, class MT, class VT>
 __device__ __forceinline__ void rowFactor(const PcgArgs<MT, VT>& a, int row, int lane, const VT* u, VT acc[3]) {
-    if (a.gL) {
-        // packed rows: only the blocks of this pass, FP16
-        const int* ptr = TR ? a.gUptr : a.gLptr;
-        const int* cl = TR ? a.gUcol : a.gLcol;
-        const __half* G = TR ? a.gU : a.gL;
-        // two of the lane's slots per round: both gathers are issued before
-        // the products, which stay in slot order
-        const int ke = ptr[row + 1];
-        for (int k = ptr[row] + lane; k < ke; k += 2 * GROUP) {
-            const int k1 = k + GROUP;
-            const bool two = k1 < ke;
-            const int c0 = cl[k], c1 = two ? cl[k1] : c0;
-            const VT x0[3] = {u[3 * c0], u[3 * c0 + 1], u[3 * c0 + 2]};
-            const VT x1[3] = {u[3 * c1], u[3 * c1 + 1], u[3 * c1 + 2]};
-            blockMulAddH(G + (size_t)9 * k, x0, acc);
-            if (two) blockMulAddH(G + (size_t)9 * k1, x1, acc);
-        }
-    } else for (int k = a.rowPtr[row] + lane; k < a.rowPtr[row + 1]; k += GROUP) {
+    for (int k = a.rowPtr[row] + lane; k < a.rowPtr[row + 1]; k += GROUP) {
         int c = a.col[k];
         if (TR ? c < row : c > row) continue;
         VT xv[3] = {u[3 * c], u[3 * c + 1], u[3 * c + 2]};
@@ -928,91 +922,34 @@ __device__ bool factorCachedPasses(const PcgArgs<MT, VT>& a, const RowCache<MT>&
     return true;
 }
 
-// acc = (A u)_row without the diagonal extras; every lane of the group gets the sum
-template <class MT, class VT>
-__device__ __forceinline__ void rowAx(const PcgArgs<MT, VT>& a, const RowIter& it, int row, const VT* u, VT acc[3]) {
-    if (row < a.nv) rowSpmv(a, row, it.lane, u, acc);
-    groupReduce3(acc);
-}
-
-// out = M^-1 w for the factor, with tmp = S w already written by the rows'
-// owners in the pass before: barrier, t = G tmp, barrier, out = S^T G^T t.
-// Ends without a barrier; false on timeout.
-template <class MT, class VT>
-__device__ bool factorPasses(const PcgArgs<MT, VT>& a, const RowIter& it, const VT* tmp, VT* out, unsigned& ep) {
-    const unsigned nb = gridDim.x;
-    const int q = it.lane;
-    if (!gridBarrier(a.bar, a.flag, nb, ep)) return false;
-    for (int base = it.first; base < a.nv; base += it.stride) {
-        int row = base + it.grp;
-        bool active = row < a.nv;
-        VT acc[3] = {VT(0), VT(0), VT(0)};
-        if (active) rowFactor<false>(a, row, it.lane, tmp, acc);
-        groupReduce3(acc);
-        // lanes 0, 1, 2 of the group store components 0, 1, 2
-        if (active && q < 3) a.t[3 * row + q] = q == 0 ? acc[0] : (q == 1 ? acc[1] : acc[2]);
-    }
-    if (!gridBarrier(a.bar, a.flag, nb, ep)) return false;
-    for (int base = it.first; base < a.nv; base += it.stride) {
-        int row = base + it.grp;
-        bool active = row < a.nv;
-        VT acc[3] = {VT(0), VT(0), VT(0)};
-        if (active) rowFactor<true>(a, row, it.lane, (const VT*)a.t, acc);
-        groupReduce3(acc);
-        if (active && q < 3) {
-            // component q of S^T y (S lower triangular)
-            const double* S = a.S + 9 * (size_t)row;
-            const double y0 = acc[0], y1 = acc[1], y2 = acc[2];
-            out[3 * row + q] = (VT)(q == 0 ? S[0] * y0 + S[3] * y1 + S[6] * y2 : (q == 1 ? S[4] * y1 + S[7] * y2 : S[8] * y2));
-        }
-    }
-    return true;
-}
-
-// MINB: blocks per SM the compiler must fit (registers: 64 per thread for
-// 2, the build of the single-pass kernel and of the two-block streaming
-// kernel); 3 and 4 for the streaming builds that trade register spills for
-// 48 or 64 resident warps
-template <class MT, class VT, bool LEARNED, bool CACHED, int MINB = 2>
-__global__ void __launch_bounds__(PB, MINB) pcgPipelinedKernel(PcgArgs<MT, VT> a) {
+// The single-pass launch: a block owns the same rows for the whole solve.
+template <class MT, class VT, bool LEARNED>
+__global__ void __launch_bounds__(PB, 2) pcgPipelinedKernel(PcgArgs<MT, VT> a) {
     extern __shared__ __align__(16) unsigned char pipeSmem[];
-    // In a single-pass launch (CACHED) the block's matrix rows and its rows'
-    // recurrence vectors live in shared memory: only the gathered vectors
-    // (u once; m, and with a factor S w and t, every iteration), the partial
-    // sums and the solution at the end touch global memory.  Lanes 0, 1, 2
-    // of a row's group update components 0, 1, 2 of the row's vectors.
+    // The block's matrix rows and its rows' recurrence vectors live in shared
+    // memory: only the gathered vectors (u once; m, and with a factor S w and
+    // t, every iteration), the partial sums and the solution at the end touch
+    // global memory.  Lanes 0, 1, 2 of a row's group update components 0, 1, 2
+    // of the row's vectors.
     const unsigned nb = gridDim.x;
     unsigned ep = 0;
-    const int nv = a.nv;
-    const RowIter it = CACHED ? RowIter(a.nv, a.rowsPerBlock) : RowIter();
-    const int rEnd = CACHED ? it.limit : a.nv;  // rows this thread's loops cover end here
+    const RowIter it(a.nv, a.rowsPerBlock);
+    const int rEnd = it.limit;  // rows this thread's loops cover end here
     const int q = it.lane;  // the component this lane updates (q < 3)
-    RowCache<MT> rc{};
-    VT* sv = nullptr;
-    if (CACHED) {
-        rc = loadRowCache<MT, VT, LEARNED>(a, pipeSmem);
-        const bool cacheG = LEARNED && a.cacheG != 0;
-        sv = reinterpret_cast<VT*>(pipeSmem + smemLayout(a.sliceMax, a.dynCap, cacheG, (int)sizeof(MT), (int)sizeof(VT)).state);
-    }
+    const RowCache<MT> rc = loadRowCache<MT, VT, LEARNED>(a, pipeSmem);
+    VT* const sv = reinterpret_cast<VT*>(
+        pipeSmem + smemLayout(a.sliceMax, a.dynCap, LEARNED && a.cacheG != 0, (int)sizeof(MT), (int)sizeof(VT)).state);
     // component q of own-row vector k (0 x, 1 r, 2 u, 3 w, 4 z, 5 q, 6 s, 7 p)
-    auto V = [&](int k, int row) -> VT& {
-        if (CACHED) return sv[(k * ROWS_PER_BLOCK + (row - rc.row0)) * 3 + q];
-        VT* g = k == 0 ? a.x : k == 1 ? a.r : k == 2 ? a.u : k == 3 ? a.w : k == 4 ? a.z : k == 5 ? a.q : k == 6 ? a.s : a.p;
-        return g[3 * row + q];
-    };
-    VT* const ownM = CACHED ? sv + 8 * ROWS_PER_BLOCK * 3 : nullptr;  // the rows' own m (shared copy)
-    VT* const ownU = CACHED ? sv + 2 * ROWS_PER_BLOCK * 3 : nullptr;
-    auto Ax = [&](int row, const VT* u, VT acc[3]) {
-        if (CACHED) rowAxCached(a, rc, it, row, u, acc);
-        else rowAx(a, it, row, u, acc);
-    };
+    auto V = [&](int k, int row) -> VT& { return sv[(k * ROWS_PER_BLOCK + (row - rc.row0)) * 3 + q]; };
+    VT* const ownM = sv + 8 * ROWS_PER_BLOCK * 3;  // the rows' own m (shared copy)
+    VT* const ownU = sv + 2 * ROWS_PER_BLOCK * 3;
     auto pick = [&](const VT v[3]) { return q == 0 ? v[0] : (q == 1 ? v[1] : v[2]); };
     // component q of D v for a row's 3x3 block D (row-major), v given whole
     auto rowDot = [&](const double* D, const VT v[3]) {
         return (VT)(D[3 * q] * (double)v[0] + D[3 * q + 1] * (double)v[1] + D[3 * q + 2] * (double)v[2]);
     };
-    auto dexRow = [&](int row) { return CACHED ? rc.dex + 9 * (row - rc.row0) : a.diagExtra + 9 * (size_t)row; };
-    auto blkRow = [&](int row) { return CACHED ? rc.blk + 9 * (row - rc.row0) : a.Dinv + 9 * (size_t)row; };
+    auto dexRow = [&](int row) { return rc.dex + 9 * (row - rc.row0); };
+    auto blkRow = [&](int row) { return rc.blk + 9 * (row - rc.row0); };
     // the group's three components of v (held by lanes 0, 1, 2); every lane calls
     auto share3 = [&](VT v, VT out[3]) {
         out[0] = __shfl_sync(0xffffffffu, v, 0, GROUP);
@@ -1029,10 +966,10 @@ __global__ void __launch_bounds__(PB, MINB) pcgPipelinedKernel(PcgArgs<MT, VT> a
         if (!LEARNED) {
             const VT mq = rowDot(blkRow(row), v);
             mOut[3 * row + q] = mq;
-            if (CACHED) ownM[3 * (row - rc.row0) + q] = mq;
+            ownM[3 * (row - rc.row0) + q] = mq;
         } else {
             // lower triangular
-            const double* S = CACHED ? rc.blk + 9 * (row - rc.row0) : a.S + 9 * (size_t)row;
+            const double* S = rc.blk + 9 * (row - rc.row0);
             const double v0 = v[0], v1 = v[1], v2 = v[2];
             sw[3 * row + q] = (VT)(q == 0 ? S[0] * v0 : (q == 1 ? S[3] * v0 + S[4] * v1 : S[6] * v0 + S[7] * v1 + S[8] * v2));
         }
@@ -1062,13 +999,7 @@ __global__ void __launch_bounds__(PB, MINB) pcgPipelinedKernel(PcgArgs<MT, VT> a
             precondRow(row, active, rv, nullptr);
         }
     }
-    if (LEARNED) {
-        if (CACHED) {
-            if (!factorCachedPasses(a, rc, it, (const VT*)sw, a.u, ownU, ep)) return;
-        } else if (!factorPasses(a, it, (const VT*)sw, a.u, ep)) {
-            return;
-        }
-    }
+    if (LEARNED && !factorCachedPasses(a, rc, it, (const VT*)sw, a.u, ownU, ep)) return;
     if (!gridBarrier(a.bar, a.flag, nb, ep)) return;
     // w = A u, m = M w, gamma = (r,u), delta = (w,u)
     double g = 0, dl = 0;
@@ -1076,10 +1007,10 @@ __global__ void __launch_bounds__(PB, MINB) pcgPipelinedKernel(PcgArgs<MT, VT> a
         const int row = base + it.grp;
         const bool active = row < rEnd;
         VT acc[3] = {VT(0), VT(0), VT(0)};
-        Ax(row, (const VT*)a.u, acc);
+        rowAxCached(a, rc, it, row, (const VT*)a.u, acc);
         VT wq = VT(0);
         if (active && q < 3) {
-            const VT* uOwn = CACHED ? ownU + 3 * (row - rc.row0) : a.u + 3 * row;
+            const VT* uOwn = ownU + 3 * (row - rc.row0);
             const VT uo[3] = {uOwn[0], uOwn[1], uOwn[2]};
             wq = pick(acc) + rowDot(dexRow(row), uo);
             V(3, row) = wq;
@@ -1093,13 +1024,7 @@ __global__ void __launch_bounds__(PB, MINB) pcgPipelinedKernel(PcgArgs<MT, VT> a
     }
     blockReduce3(rr, g, dl);
     if (threadIdx.x == 0) { part(0, 0)[blockIdx.x] = rr; part(0, 1)[blockIdx.x] = g; part(0, 2)[blockIdx.x] = dl; }
-    if (LEARNED) {
-        if (CACHED) {
-            if (!factorCachedPasses(a, rc, it, (const VT*)sw, a.mA, ownM, ep)) return;
-        } else if (!factorPasses(a, it, (const VT*)sw, a.mA, ep)) {
-            return;
-        }
-    }
+    if (LEARNED && !factorCachedPasses(a, rc, it, (const VT*)sw, a.mA, ownM, ep)) return;
     {
         double sums[3];
         if (!gridBarrierSum<3>(a.bar, a.flag, nb, ep, part(0, 0), PIPE_PMAX, sums)) return;
@@ -1123,10 +1048,10 @@ __global__ void __launch_bounds__(PB, MINB) pcgPipelinedKernel(PcgArgs<MT, VT> a
             const int row = base + it.grp;
             const bool active = row < rEnd;
             VT acc[3] = {VT(0), VT(0), VT(0)};
-            Ax(row, mCur, acc);
+            rowAxCached(a, rc, it, row, mCur, acc);
             VT wq = VT(0);
             if (active && q < 3) {
-                const VT* mOwn = CACHED ? ownM + 3 * (row - rc.row0) : mCur + 3 * row;
+                const VT* mOwn = ownM + 3 * (row - rc.row0);
                 const VT mo[3] = {mOwn[0], mOwn[1], mOwn[2]};
                 const VT zv = pick(acc) + rowDot(dexRow(row), mo) + bt * V(4, row);
                 const VT qv = pick(mo) + bt * V(5, row);
@@ -1151,13 +1076,7 @@ __global__ void __launch_bounds__(PB, MINB) pcgPipelinedKernel(PcgArgs<MT, VT> a
         if (threadIdx.x == 0) { part(set, 0)[blockIdx.x] = lrr; part(set, 1)[blockIdx.x] = lg; part(set, 2)[blockIdx.x] = ld; }
         // the factor's m is replaced only in its last pass, two barriers
         // after every row read it
-        if (LEARNED) {
-            if (CACHED) {
-                if (!factorCachedPasses(a, rc, it, (const VT*)sw, mNext, ownM, ep)) return;
-            } else if (!factorPasses(a, it, (const VT*)sw, mNext, ep)) {
-                return;
-            }
-        }
+        if (LEARNED && !factorCachedPasses(a, rc, it, (const VT*)sw, mNext, ownM, ep)) return;
         double sums[3];
         if (!gridBarrierSum<3>(a.bar, a.flag, nb, ep, part(set, 0), PIPE_PMAX, sums)) return;
         gPrev = g;
@@ -1167,17 +1086,472 @@ __global__ void __launch_bounds__(PB, MINB) pcgPipelinedKernel(PcgArgs<MT, VT> a
         if (rr < thr) { status = 1; break; }
         if (iter >= a.maxIter || !isfinite(rr)) { status = 2; break; }
     }
-    if (CACHED) {
-        // the solution leaves shared memory
-        for (int base = it.first; base < rEnd; base += it.stride) {
-            const int row = base + it.grp;
-            if (row < rEnd && q < 3) a.x[3 * row + q] = V(0, row);
-        }
+    // the solution leaves shared memory
+    for (int base = it.first; base < rEnd; base += it.stride) {
+        const int row = base + it.grp;
+        if (row < rEnd && q < 3) a.x[3 * row + q] = V(0, row);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.scal[3] = rr;
         a.scal[4] = iter;
         a.scal[6] = rhs2;
+        atomicCAS(a.flag, 0, status);  // a barrier timeout (3) stands
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Streaming pipelined PCG, for systems whose rows do not fit the chip's shared
+// memory: the recurrences of pcgPipelinedKernel over matrices in tiles.
+//
+// A warp takes 8 rows at a time, 4 lanes to a row.  In block-CSR order each of
+// a lane's nine loads of a block touched lines of all 8 rows, at 40 registers
+// with 48 warps, and the loads waited for one another.  The tiles hold the
+// blocks of one step of the warp lane by lane (16 bytes per lane and load), so
+// every load is one contiguous run; a lane without a block has column -1 and
+// reads no values.  The gathered vectors have 4 entries per row, one 32-byte
+// load each.  A block owns a contiguous run of tiles, the same in every pass,
+// and keeps its rows' eight recurrence vectors in shared memory where they fit
+// (STREAM_STATE_BYTES): on the 64-cube pile 54 MB less traffic per iteration.
+// Sums run in the order of the block-CSR rows.
+//
+// Bound by memory latency within L2 and by memory beyond it.  Measured per
+// solve on a B200, block-CSR rows -> tiles: 13x81 twist (FP64, block-Jacobi, 427
+// iterations) 9.3 -> 4.5 ms, 27-cube pile (FP32 blocks) 16.7 -> 7.9 ms, with the
+// factor 16.4 -> 10.9 ms, 64-cube pile 27.9 -> 15.0 ms, with the factor 25.9 ->
+// 23.8 ms.
+// ---------------------------------------------------------------------------
+// Warps per block, one block per SM.  A system within L2 waits for latency:
+// 16 warps, two steps of a row in flight (128 registers).  One beyond it waits
+// for memory: 24 warps, one step each, the next tile fetched ahead (80
+// registers).  Measured, in ms per solve: 64-cube pile 14.9 against 16.7 with 16
+// warps, with the factor 23.8 against 26.7; 13x81 twist 4.5 without the fetch
+// and the priorities against 5.4 with them.
+constexpr int streamWarps(bool beyond) { return beyond ? 24 : 16; }
+// Beyond when an iteration's data exceed this share of L2 (63 MB): 27-cube pile,
+// 45 MB, 7.9 ms within and 9.2 beyond; with the factor, 75 MB, 11.8 and 10.9.
+constexpr double STREAM_L2_SHARE = 0.5;
+constexpr size_t STREAM_STATE_BYTES = 192 * 1024;  // recurrence vectors in shared memory, per SM
+
+// fetch [p, p + bytes) into L2 (both multiples of 16)
+__device__ __forceinline__ void prefetchL2(const void* p, int bytes, uint64_t pol) {
+    asm volatile("cp.async.bulk.prefetch.L2.global.L2::cache_hint [%0], %1, %2;" ::"l"(p), "r"(bytes), "l"(pol));
+}
+
+// entries 0-2 of row c of a padded vector, in one 32-byte load
+__device__ __forceinline__ void gather3(const double* u, int c, double x[3]) {
+    double pad;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(pad) : "l"(u + 4 * (size_t)c));
+}
+
+// L2 priority of streamed data in a system beyond L2: the matrix goes first, so
+// that the factor and the vectors stay
+template <bool FIRST>
+__device__ __forceinline__ uint64_t streamPolicy() {
+    uint64_t p;
+    if (FIRST) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    else asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+// constant data, read once per pass: past L1
+__device__ __forceinline__ uint4 streamLoad16(const void* p, uint64_t pol) {
+    uint4 v;
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ void streamLoad(const float* p, uint64_t pol, float& v) {
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+}
+__device__ __forceinline__ void streamLoad(const double* p, uint64_t pol, double& v) {
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
+}
+__device__ __forceinline__ void streamLoad(const unsigned short* p, uint64_t pol, unsigned short& v) {
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(v) : "l"(p), "l"(pol));
+}
+__device__ __forceinline__ int streamLoad(const int* p, uint64_t pol) {
+    int v;
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
+    return v;
+}
+
+// one lane's block of a step
+template <class T>
+struct SellBlock;
+template <>
+struct SellBlock<float> {
+    uint4 a, b;
+    float c;
+    __device__ __forceinline__ void load(const void* step, int lane, uint64_t pol) {
+        a = streamLoad16((const uint4*)step + lane, pol);
+        b = streamLoad16((const uint4*)step + 32 + lane, pol);
+        streamLoad((const float*)step + 256 + lane, pol, c);
+    }
+    __device__ __forceinline__ void mulAdd(const double x[3], double acc[3]) const {
+        const float B[9] = {__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), __uint_as_float(a.w), __uint_as_float(b.x),
+                            __uint_as_float(b.y), __uint_as_float(b.z), __uint_as_float(b.w), c};
+        blockMulAdd(B, x, acc);
+    }
+};
+template <>
+struct SellBlock<double> {
+    uint4 a[4];
+    double e;
+    __device__ __forceinline__ void load(const void* step, int lane, uint64_t pol) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) a[k] = streamLoad16((const uint4*)step + 32 * k + lane, pol);
+        streamLoad((const double*)step + 256 + lane, pol, e);
+    }
+    __device__ __forceinline__ void mulAdd(const double x[3], double acc[3]) const {
+        double B[9];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            B[2 * k] = __hiloint2double((int)a[k].y, (int)a[k].x);
+            B[2 * k + 1] = __hiloint2double((int)a[k].w, (int)a[k].z);
+        }
+        B[8] = e;
+        blockMulAdd(B, x, acc);
+    }
+};
+template <>
+struct SellBlock<__half> {
+    uint4 a;
+    unsigned short b;
+    __device__ __forceinline__ void load(const void* step, int lane, uint64_t pol) {
+        a = streamLoad16((const uint4*)step + lane, pol);
+        streamLoad((const unsigned short*)step + 256 + lane, pol, b);
+    }
+    __device__ __forceinline__ void mulAdd(const double x[3], double acc[3]) const {
+        const unsigned w[4] = {a.x, a.y, a.z, a.w};
+        __half B[9];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            B[2 * k] = __ushort_as_half((unsigned short)(w[k] & 0xffffu));
+            B[2 * k + 1] = __ushort_as_half((unsigned short)(w[k] >> 16));
+        }
+        B[8] = __ushort_as_half(b);
+        blockMulAddH(B, x, acc);
+    }
+};
+
+// A warp's way through its tiles of one pass: the step ranges of the current
+// and the next tile.  Beyond L2, the next tile's columns and values are fetched
+// into it by one bulk prefetch each while a tile is worked on.
+template <bool BEYOND>
+struct SellCursor {
+    static constexpr int W = streamWarps(BEYOND);
+    int s, n, sn, nn;
+    __device__ __forceinline__ void start(const SellView& m, int tile, int hi) {
+        s = n = 0;
+        if (tile < hi) { s = __ldcg(m.tile + tile); n = __ldcg(m.tile + tile + 1) - s; }
+        sn = nn = 0;
+        tile += W;
+        if (tile < hi) { sn = __ldcg(m.tile + tile); nn = __ldcg(m.tile + tile + 1) - sn; }
+    }
+    template <class T, bool FIRST>
+    __device__ __forceinline__ void prefetch(const SellView& m, int s, int n) const {
+        if (BEYOND && n > 0 && (threadIdx.x & 31) == 0) {
+            const uint64_t pol = streamPolicy<FIRST>();
+            prefetchL2(m.col + (size_t)s * 32, n * 128, pol);
+            prefetchL2((const char*)m.val + (size_t)s * (288 * sizeof(T)), n * (int)(288 * sizeof(T)), pol);
+        }
+    }
+    // at the end of a tile: on to the next, and the range after it
+    __device__ __forceinline__ void next(const SellView& m, int tile, int hi) {
+        s = sn; n = nn;
+        sn = nn = 0;
+        tile += 2 * W;
+        if (tile < hi) { sn = __ldcg(m.tile + tile); nn = __ldcg(m.tile + tile + 1) - sn; }
+    }
+};
+
+// acc += (M u)_row over the tile's static blocks of this lane.  A round of two
+// steps (one of FP64 blocks, or beyond L2: registers) requests its gathers and values, and
+// the next round's columns, before the products.
+template <class T, bool BEYOND, bool FIRST>
+__device__ __forceinline__ void sellRow(const SellView& m, int s0, int n, const double* u, double acc[3]) {
+    constexpr int R = BEYOND || sizeof(T) == 8 ? 1 : 2;
+    int wl = threadIdx.x & 31;
+    asm volatile("" : "+r"(wl));  // see StreamPlace::first
+    int left = n;
+    const uint64_t pol = streamPolicy<BEYOND && FIRST>();
+    const int* cp = m.col + (size_t)s0 * 32 + wl;
+    const char* vp = (const char*)m.val + (size_t)s0 * (288 * sizeof(T));
+    int c[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) c[j] = j < left ? streamLoad(cp + 32 * j, pol) : -1;
+#pragma unroll 1
+    for (; left > 0; left -= R) {
+        SellBlock<T> b[R];
+        double x[R][3];
+        int nx[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+            if (c[j] >= 0) { b[j].load(vp + j * 288 * sizeof(T), wl, pol); gather3(u, c[j], x[j]); }
+        cp += 32 * R;
+        vp += R * 288 * sizeof(T);
+#pragma unroll
+        for (int j = 0; j < R; ++j) nx[j] = R + j < left ? streamLoad(cp + 32 * j, pol) : -1;
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            if (c[j] >= 0) b[j].mulAdd(x[j], acc);
+            c[j] = nx[j];
+        }
+    }
+}
+
+// Where a thread of the streaming kernel works: its warp's first tile and the
+// block's last, the component it updates, its row in a tile, and the
+// recurrence vectors, tile by tile: the 24 entries of x, then r, u, w, z, q,
+// s, p (in shared or global memory).
+enum StreamVec { SV_X, SV_R, SV_U, SV_W, SV_Z, SV_Q, SV_S, SV_P };
+struct StreamPlace {
+    int tFirst, tHi;
+    double* st;
+    // the compiler sees a new value in every pass: the passes' addresses, formed
+    // once before the iterations, would spill 60-100 registers
+    __device__ __forceinline__ int first() const {
+        int t = tFirst;
+        asm volatile("" : "+r"(t));
+        return t;
+    }
+    __device__ __forceinline__ int q() const { return threadIdx.x & (GROUP - 1); }
+    __device__ __forceinline__ int row(int tile) const { return 8 * tile + (threadIdx.x & 31) / GROUP; }
+    // this thread's entry of vector 0 (lanes q < 3); vector k lies 24 k further
+    __device__ __forceinline__ double* own(int tile) const { return st + (ptrdiff_t)192 * tile + 3 * ((threadIdx.x & 31) / GROUP) + q(); }
+};
+
+__device__ __forceinline__ double pick3(const double v[3], int q) { return q == 0 ? v[0] : (q == 1 ? v[1] : v[2]); }
+__device__ __forceinline__ double rowDot3(const double* D, int q, const double v[3]) {
+    return D[3 * q] * v[0] + D[3 * q + 1] * v[1] + D[3 * q + 2] * v[2];
+}
+
+// The group's sum of (M u)_row over the static blocks and the contact blocks
+// (all, or with TRI < 0 / > 0 those left / right of the diagonal), in every lane
+template <class T, int TRI, bool BEYOND, class MT>
+__device__ __forceinline__ void streamRow(const PcgArgs<MT, double>& a, const SellView& m, const SellCursor<BEYOND>& cur, const float* factor, const MT* matrix,
+                                          int row, const double* u, double acc[3]) {
+    acc[0] = acc[1] = acc[2] = 0.0;
+    sellRow<T, BEYOND, TRI == 0>(m, cur.s, cur.n, u, acc);
+    if (a.dRowS && row < a.nv) {
+#pragma unroll 1
+        for (int k = a.dRowS[row] + (threadIdx.x & (GROUP - 1)), ke = a.dRowE[row]; k < ke; k += GROUP) {
+            const int c = a.dCol[k];
+            if ((TRI < 0 && c >= row) || (TRI > 0 && c <= row)) continue;
+            double xv[3];
+            gather3(u, c, xv);
+            if (TRI == 0) blockMulAdd(matrix + (size_t)9 * k, xv, acc);
+            else blockMulAdd(factor + (size_t)9 * k, xv, acc);
+        }
+    }
+    groupReduce3(acc);
+}
+
+// From component q of v in each lane: block-Jacobi Dinv v, or with a factor
+// S v (lower triangular), the input of the factor's first pass.  The fourth
+// lane writes the pad, so that whole sectors are written.
+template <bool LEARNED, class MT>
+__device__ __forceinline__ double streamPrecond(const PcgArgs<MT, double>& a, int row, double vq, double* out) {
+    const int q = threadIdx.x & (GROUP - 1);
+    const double v[3] = {__shfl_sync(0xffffffffu, vq, 0, GROUP), __shfl_sync(0xffffffffu, vq, 1, GROUP), __shfl_sync(0xffffffffu, vq, 2, GROUP)};
+    double o = 0.0;
+    if (row < a.nv) {
+        if (q < 3) {
+            if (!LEARNED) {
+                o = rowDot3(a.Dinv + 9 * (size_t)row, q, v);
+            } else {
+                const double* S = a.S + 9 * (size_t)row + 3 * q;
+                const double p1 = S[1] * v[1], p2 = S[2] * v[2];
+                o = S[0] * v[0] + (q > 0 ? p1 : 0.0) + (q > 1 ? p2 : 0.0);
+            }
+        }
+        out[4 * (size_t)row + q] = o;
+    }
+    return o;
+}
+
+// out = S^T G^T G (S w), with S w in g2 already; ends without a barrier.  The
+// result is also the rows' u where ownU.  False on a barrier timeout.
+template <class FT, bool BEYOND, class MT>
+__device__ __forceinline__ bool streamFactor(const PcgArgs<MT, double>& a, const StreamPlace& at, double* out, bool ownU, unsigned& ep) {
+    const int q = at.q();
+    constexpr int W = streamWarps(BEYOND);
+    SellCursor<BEYOND> cur;
+    cur.start(a.sL, at.first(), at.tHi);
+    cur.template prefetch<FT, false>(a.sL, cur.s, cur.n);
+    if (!gridBarrier(a.bar, a.flag, gridDim.x, ep)) return false;
+    for (int tile = at.first(); tile < at.tHi; tile += W) {
+        const int row = at.row(tile);
+        double acc[3];
+        cur.template prefetch<FT, false>(a.sL, cur.sn, cur.nn);
+        streamRow<FT, -1, BEYOND>(a, a.sL, cur, a.gD, (const MT*)nullptr, row, a.g2, acc);
+        cur.next(a.sL, tile, at.tHi);
+        if (row < a.nv) a.g3[4 * (size_t)row + q] = q < 3 ? pick3(acc, q) : 0.0;
+    }
+    cur.start(a.sU, at.first(), at.tHi);
+    cur.template prefetch<FT, false>(a.sU, cur.s, cur.n);
+    if (!gridBarrier(a.bar, a.flag, gridDim.x, ep)) return false;
+    for (int tile = at.first(); tile < at.tHi; tile += W) {
+        const int row = at.row(tile);
+        double acc[3];
+        cur.template prefetch<FT, false>(a.sU, cur.sn, cur.nn);
+        streamRow<FT, 1, BEYOND>(a, a.sU, cur, a.gD, (const MT*)nullptr, row, a.g3, acc);
+        cur.next(a.sU, tile, at.tHi);
+        if (row < a.nv) {
+            double o = 0.0;
+            if (q < 3) {
+                // component q of S^T y
+                const double* S = a.S + 9 * (size_t)row + 4 * q;
+                o = S[0] * pick3(acc, q);
+                if (q < 2) o += S[3] * (q == 0 ? acc[1] : acc[2]);
+                if (q < 1) o += S[6] * acc[2];
+                if (ownU) at.own(tile)[24 * SV_U] = o;
+            }
+            out[4 * (size_t)row + q] = o;
+        }
+    }
+    return true;
+}
+
+template <class MT, class FT, bool LEARNED, bool BEYOND>
+__global__ void __launch_bounds__(32 * streamWarps(BEYOND), 1) pcgStreamKernel(PcgArgs<MT, double> a) {
+    constexpr int W = streamWarps(BEYOND);
+    extern __shared__ __align__(16) unsigned char pipeSmem[];
+    __shared__ double sc[3];  // the last gamma and alpha, and the stopping threshold
+    const unsigned nb = gridDim.x;
+    unsigned ep = 0;
+    const int nTiles = (a.nv + 7) / 8;
+    StreamPlace at;
+    const int tLo = (int)((long long)nTiles * blockIdx.x / nb);
+    at.tHi = (int)((long long)nTiles * (blockIdx.x + 1) / nb);
+    at.tFirst = tLo + (threadIdx.x >> 5);
+    at.st = a.resident ? reinterpret_cast<double*>(pipeSmem) - 192 * (ptrdiff_t)tLo : a.state;
+    const int q = at.q();
+    auto part = [&](int set, int k) { return a.pp + (size_t)(3 * set + k) * PIPE_PMAX; };
+    // x = 0, r = b, u = M r (gathered from g1); the recurrence vectors start at 0
+    double s0 = 0, s1 = 0, s2 = 0;  // this thread's shares of r.r, gamma = (r,u), delta = (w,u)
+    for (int tile = at.first(); tile < at.tHi; tile += W) {
+        const int row = at.row(tile);
+        double rq = 0.0;
+        if (row < a.nv && q < 3) {
+            double* v = at.own(tile);
+            v[24 * SV_X] = v[24 * SV_Z] = v[24 * SV_Q] = v[24 * SV_S] = v[24 * SV_P] = 0.0;
+            rq = a.b[3 * (size_t)row + q];
+            v[24 * SV_R] = rq;
+            s0 += rq * rq;
+        }
+        const double u = streamPrecond<LEARNED>(a, row, rq, LEARNED ? a.g2 : a.g1);
+        if (!LEARNED && row < a.nv && q < 3) at.own(tile)[24 * SV_U] = u;
+    }
+    if (LEARNED && !streamFactor<FT, BEYOND>(a, at, a.g1, true, ep)) return;
+    if (!gridBarrier(a.bar, a.flag, nb, ep)) return;
+    // w = A u, m = M w
+    SellCursor<BEYOND> cur;
+    cur.start(a.sA, at.first(), at.tHi);
+    for (int tile = at.first(); tile < at.tHi; tile += W) {
+        const int row = at.row(tile);
+        double acc[3];
+        streamRow<MT, 0, BEYOND>(a, a.sA, cur, (const float*)nullptr, a.dVal, row, a.g1, acc);
+        cur.next(a.sA, tile, at.tHi);
+        double wq = 0.0;
+        if (row < a.nv && q < 3) {
+            double uo[3];
+            gather3(a.g1, row, uo);
+            wq = pick3(acc, q) + rowDot3(a.diagExtra + 9 * (size_t)row, q, uo);
+            double* v = at.own(tile);
+            v[24 * SV_W] = wq;
+            const double uq = v[24 * SV_U];
+            s1 += v[24 * SV_R] * uq;
+            s2 += wq * uq;
+        }
+        streamPrecond<LEARNED>(a, row, wq, LEARNED ? a.g2 : a.g0);
+    }
+    blockReduce3(s0, s1, s2);
+    if (threadIdx.x == 0) { part(0, 0)[blockIdx.x] = s0; part(0, 1)[blockIdx.x] = s1; part(0, 2)[blockIdx.x] = s2; }
+    if (LEARNED && !streamFactor<FT, BEYOND>(a, at, a.g0, false, ep)) return;
+    double sums[3];  // r.r, gamma, delta
+    cur.start(a.sA, at.first(), at.tHi);
+    if (!gridBarrierSum<3>(a.bar, a.flag, nb, ep, part(0, 0), PIPE_PMAX, sums)) return;
+    if (threadIdx.x == 0) {
+        sc[0] = sc[1] = 1.0;
+        sc[2] = fmax(a.tol * a.tol * sums[0], 2.2250738585072014e-308);
+        if (blockIdx.x == 0) a.scal[6] = sums[0];
+    }
+    __syncthreads();
+    int iter = 0;
+    int status = (sums[0] == 0.0 || sums[0] < sc[2]) ? 1 : 0;
+    while (status == 0) {
+        const double g = sums[1];
+        const double bt = iter == 0 ? 0.0 : g / sc[0];
+        const double den = iter == 0 ? sums[2] : sums[2] - bt * g / sc[1];
+        if (!(den != 0.0) || !isfinite(den)) { status = 2; break; }  // breakdown: the caller's true residual decides
+        const double al = g / den;
+        const double* mCur = (LEARNED || (iter & 1) == 0) ? a.g0 : a.g1;
+        s0 = s1 = s2 = 0.0;
+        for (int tile = at.first(); tile < at.tHi; tile += W) {
+            const int row = at.row(tile);
+            double acc[3];
+            cur.template prefetch<MT, true>(a.sA, cur.sn, cur.nn);
+            if (BEYOND && (threadIdx.x & 31) == 0 && tile + W < at.tHi && 8 * (tile + W) + 8 <= a.nv) {
+                const size_t o = 72 * (size_t)(tile + W);
+                const uint64_t pol = streamPolicy<false>();
+                prefetchL2(a.diagExtra + o, 576, pol);
+                prefetchL2((LEARNED ? a.S : a.Dinv) + o, 576, pol);
+            }
+            streamRow<MT, 0, BEYOND>(a, a.sA, cur, (const float*)nullptr, a.dVal, row, mCur, acc);
+            cur.next(a.sA, tile, at.tHi);
+            double wq = 0.0;
+            if (row < a.nv && q < 3) {
+                double mo[3];
+                gather3(mCur, row, mo);
+                double* v = at.own(tile);
+                const double zv = pick3(acc, q) + rowDot3(a.diagExtra + 9 * (size_t)row, q, mo) + bt * v[24 * SV_Z];
+                v[24 * SV_Z] = zv;
+                const double w0 = v[24 * SV_W];
+                wq = w0 - al * zv;
+                v[24 * SV_W] = wq;
+                const double sq = w0 + bt * v[24 * SV_S];
+                v[24 * SV_S] = sq;
+                const double u0 = v[24 * SV_U];
+                const double pv = u0 + bt * v[24 * SV_P];
+                v[24 * SV_P] = pv;
+                v[24 * SV_X] += al * pv;
+                const double qv = pick3(mo, q) + bt * v[24 * SV_Q];
+                v[24 * SV_Q] = qv;
+                const double uv = u0 - al * qv;
+                v[24 * SV_U] = uv;
+                const double rv = v[24 * SV_R] - al * sq;
+                v[24 * SV_R] = rv;
+                s0 += rv * rv;
+                s1 += rv * uv;
+                s2 += wq * uv;
+            }
+            streamPrecond<LEARNED>(a, row, wq, LEARNED ? a.g2 : ((iter & 1) == 0 ? a.g1 : a.g0));
+        }
+        const int set = (iter + 1) & 1;
+        blockReduce3(s0, s1, s2);
+        if (threadIdx.x == 0) {
+            part(set, 0)[blockIdx.x] = s0; part(set, 1)[blockIdx.x] = s1; part(set, 2)[blockIdx.x] = s2;
+            sc[0] = g;
+            sc[1] = al;
+        }
+        // the factor's m is replaced only in its last pass, two barriers
+        // after every row read it
+        if (LEARNED && !streamFactor<FT, BEYOND>(a, at, a.g0, false, ep)) return;
+        cur.start(a.sA, at.first(), at.tHi);
+        cur.template prefetch<MT, true>(a.sA, cur.s, cur.n);
+        if (!gridBarrierSum<3>(a.bar, a.flag, nb, ep, part(set, 0), PIPE_PMAX, sums)) return;
+        ++iter;
+        if (sums[0] < sc[2]) { status = 1; break; }
+        if (iter >= a.maxIter || !isfinite(sums[0])) { status = 2; break; }
+    }
+    // the solution leaves the state
+    for (int tile = at.first(); tile < at.tHi; tile += W) {
+        const int row = at.row(tile);
+        if (row < a.nv && q < 3) a.x[3 * (size_t)row + q] = at.own(tile)[24 * SV_X];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.scal[3] = sums[0];
+        a.scal[4] = iter;
         atomicCAS(a.flag, 0, status);  // a barrier timeout (3) stands
     }
 }
@@ -1192,53 +1566,95 @@ __global__ void zeroKernel(int n3, double* x) {
 
 }  // namespace
 
-// packed[k] = the FP16 block of slot slot[k] of G (transposed where the
-// slot is stored as ~slot: the diagonal blocks of the transposed part)
-__global__ void packFactorKernel(int n, const int* slot, const float* gS, __half* out) {
-    CIPC_KERNEL_LOOP(i, 9 * n) {
-        const int k = i / 9, e = i - 9 * k;
-        const int s = slot[k];
-        const bool tr = s < 0;
-        const int src = tr ? 3 * (e % 3) + e / 3 : e;
-        out[i] = __float2half_rn(gS[(size_t)9 * (tr ? ~s : s) + src]);
+// One warp per tile copies the tile's blocks into the layout of SellView:
+// lane l of step j holds block 4 j + l % 4 of the tile's row l / 4.  slotOf
+// lists the rows' source slots (null: the block-CSR slots themselves; ~slot:
+// the block is transposed).  Columns are written when col is given.
+template <class MT, class OT>
+__global__ void packTilesKernel(int nv, const int* ptr, const int* slotOf, const int* srcCol, const MT* src, const int* tile, int* col, OT* out) {
+    const int nTiles = (nv + 7) / 8, wl = threadIdx.x & 31;
+    const int nWarps = gridDim.x * blockDim.x / 32;
+    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) / 32; t < nTiles; t += nWarps) {
+        const int row = 8 * t + wl / GROUP;
+        int k = 0, ke = 0;
+        if (row < nv) { k = ptr[row] + (wl & (GROUP - 1)); ke = ptr[row + 1]; }
+        for (int st = tile[t], se = tile[t + 1]; st < se; ++st, k += GROUP) {
+            int c = -1;
+            if (k < ke) {
+                int s = slotOf ? slotOf[k] : k;
+                const bool tr = s < 0;
+                if (tr) s = ~s;
+                if (col) c = srcCol[s];
+                const MT* B = src + (size_t)9 * s;
+                OT* o = out + (size_t)st * 288;
+                // 16-byte runs of each lane, then the ninth values
+                constexpr int RUN = 16 / sizeof(OT);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) o[(e / RUN) * 32 * RUN + wl * RUN + e % RUN] = (OT)B[tr ? 3 * (e % 3) + e / 3 : e];
+                o[256 + wl] = (OT)B[8];
+            }
+            if (col) col[(size_t)st * 32 + wl] = c;
+        }
     }
 }
 
-// The factor's static blocks in the packed layout the streaming PCG reads
-// (rowFactor): per row the slots with column <= row (G), then those with
-// column >= row (G^T: the mirror slots, and the diagonal transposed).  The
-// index lists follow the static pattern and are built on the first call.
-static void packFactor(Ctx& c) {
+// Step offsets of the tiles of 8 rows with the given row offsets.
+static void tileOffsets(SellRows& m, int nv, const std::vector<int>& ptr) {
+    std::vector<int> tile((nv + 7) / 8 + 1, 0);
+    for (int t = 0; 8 * t < nv; ++t) {
+        int steps = 0;
+        for (int r = 8 * t; r < std::min(nv, 8 * t + 8); ++r) steps = std::max(steps, (ptr[r + 1] - ptr[r] + GROUP - 1) / GROUP);
+        tile[t + 1] = tile[t] + steps;
+    }
+    m.steps = tile.back();
+    m.tile.reserve(tile.size());
+    CIPC_CUDA(cudaMemcpy(m.tile.p, tile.data(), sizeof(int) * tile.size(), cudaMemcpyHostToDevice));
+}
+
+template <class MT, class OT>
+static void packTiles(Ctx& c, SellRows& m, const int* ptr, const int* slotOf, const MT* src) {
+    const bool first = m.col.cap == 0;
+    m.col.reserve(std::max<size_t>((size_t)32 * m.steps, 1));
+    m.val.reserve(std::max<size_t>((size_t)288 * sizeof(OT) * m.steps, 16));
+    const int nb = std::max(1, std::min(((c.nv + 7) / 8 + VB / 32 - 1) / (VB / 32), 148 * 8));
+    launch(packTilesKernel<MT, OT>, nb, VB, 0, c.s, c.nv, ptr, slotOf, (const int*)c.colIdx, src, (const int*)m.tile, first ? m.col.p : (int*)nullptr,
+           reinterpret_cast<OT*>(m.val.p));
+    CIPC_CUDA(cudaGetLastError());
+}
+
+// The static matrix and, with a factor, its static blocks in tiles: per row
+// the slots with column <= row (G), then those with column >= row (G^T: the
+// mirror slots, and the diagonal transposed).  Offsets and columns follow the
+// static pattern and are laid out on the first call; values on every call.
+template <class MT, class FT>
+static void packStream(Ctx& c, const MT* val, bool learned) {
     const int nv = c.nv;
-    if (c.nGL == 0) {
+    if (c.sellA.tile.cap == 0) tileOffsets(c.sellA, nv, c.hRowPtr);
+    packTiles<MT, MT>(c, c.sellA, c.rowPtr, nullptr, val);
+    if (!learned) return;
+    if (c.sellL.tile.cap == 0) {
         std::vector<int> col(c.nnzb);
         CIPC_CUDA(cudaMemcpy(col.data(), c.colIdx.p, sizeof(int) * c.nnzb, cudaMemcpyDeviceToHost));
-        std::vector<int> lp(nv + 1, 0), lc, ls, up(nv + 1, 0), uc, us;
-        lc.reserve(c.nnzb / 2 + nv); ls.reserve(c.nnzb / 2 + nv); uc.reserve(c.nnzb / 2 + nv); us.reserve(c.nnzb / 2 + nv);
+        std::vector<int> lp(nv + 1, 0), ls, up(nv + 1, 0), us;
+        ls.reserve(c.nnzb / 2 + nv); us.reserve(c.nnzb / 2 + nv);
         for (int r = 0; r < nv; ++r) {
             for (int k = c.hRowPtr[r]; k < c.hRowPtr[r + 1]; ++k) {
-                const int cl = col[k];
-                if (cl <= r) { lc.push_back(cl); ls.push_back(k); }
-                if (cl >= r) { uc.push_back(cl); us.push_back(cl == r ? ~k : k); }
+                if (col[k] <= r) ls.push_back(k);
+                if (col[k] >= r) us.push_back(col[k] == r ? ~k : k);
             }
-            lp[r + 1] = (int)lc.size();
-            up[r + 1] = (int)uc.size();
+            lp[r + 1] = (int)ls.size();
+            up[r + 1] = (int)us.size();
         }
         auto up_ = [&](DBuf<int>& d, const std::vector<int>& h) {
             d.reserve(std::max<size_t>(h.size(), 1));
             if (!h.empty()) CIPC_CUDA(cudaMemcpy(d.p, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice));
         };
-        up_(c.gLptr, lp); up_(c.gLcol, lc); up_(c.gLslot, ls); up_(c.gUptr, up); up_(c.gUcol, uc); up_(c.gUslot, us);
-        c.nGL = (int)lc.size();
-        c.nGU = (int)uc.size();
-        c.gLval.reserve(9 * (size_t)std::max(1, c.nGL));
-        c.gUval.reserve(9 * (size_t)std::max(1, c.nGU));
+        up_(c.sellL.ptr, lp); up_(c.sellL.slot, ls); up_(c.sellU.ptr, up); up_(c.sellU.slot, us);
+        tileOffsets(c.sellU, nv, up);
+        tileOffsets(c.sellL, nv, lp);
     }
-    const int vb = std::max(1, std::min((9 * c.nGL + VB - 1) / VB, 148 * 16));
-    launch(packFactorKernel, vb, VB, 0, c.s, c.nGL, (const int*)c.gLslot, (const float*)c.mpGS, reinterpret_cast<__half*>(c.gLval.p));
-    const int ub = std::max(1, std::min((9 * c.nGU + VB - 1) / VB, 148 * 16));
-    launch(packFactorKernel, ub, VB, 0, c.s, c.nGU, (const int*)c.gUslot, (const float*)c.mpGS, reinterpret_cast<__half*>(c.gUval.p));
-    CIPC_CUDA(cudaGetLastError());
+    packTiles<float, FT>(c, c.sellL, c.sellL.ptr, c.sellL.slot, (const float*)c.mpGS);
+    packTiles<float, FT>(c, c.sellU, c.sellU.ptr, c.sellU.slot, (const float*)c.mpGS);
 }
 
 void buildRhs(Ctx& c) {
@@ -1315,7 +1731,7 @@ static int runPcg(Ctx& c, const MT* val, const MT* dval, const VT* b, VT* x, VT*
 
 constexpr int PMAX = 1024;  // max blocks of the persistent PCG
 
-// Blocks per SM of the persistent PCG: CIPC_PCG_BLOCKS_PER_SM (1-8) or 2.
+// Blocks per SM of the textbook kernel: CIPC_PCG_BLOCKS_PER_SM (1-8) or 2.
 static int pcgBlocksPerSm() {
     static int v = -1;
     if (v < 0) {
@@ -1334,20 +1750,7 @@ static bool pcgClassic() {
     return v == 1;
 }
 
-// Blocks per SM of the streaming kernel's build: 3 by default (48 resident
-// warps for a few register spills: measured 10-24 % faster per solve on the
-// pile than two blocks per SM); CIPC_PCG_OCC=2 or 4 selects the other builds.
-static int pcgOcc() {
-    static int v = -1;
-    if (v < 0) {
-        const char* e = std::getenv("CIPC_PCG_OCC");
-        v = e ? std::atoi(e) : 3;
-        if (v != 2 && v != 4) v = 3;
-    }
-    return v;
-}
-
-// CIPC_PCG_NOPACK=1 keeps the streaming kernel on the slot-aligned FP32 factor.
+// CIPC_PCG_NOPACK=1 keeps the streaming kernel's factor in FP32.
 static bool pcgNoPack() {
     static int v = -1;
     if (v < 0) { const char* e = std::getenv("CIPC_PCG_NOPACK"); v = (e && *e == '1') ? 1 : 0; }
@@ -1361,8 +1764,6 @@ static bool pcgNoCache() {
     return v == 1;
 }
 
-// Largest number of static slots over the row ranges the cached kernel's
-// blocks own (computed once per context from the static pattern).
 // CIPC_DEBUG_PCG=1 prints every inner solve and fallback to stderr.
 static bool debugPcg() {
     static int v = -1;
@@ -1401,7 +1802,7 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
         const int nbRows = (c.nv + rows - 1) / rows;
         a.rowsPerBlock = rows;
         a.sliceMax = pcgSliceMax(c, rows);
-        const void* fn = (const void*)pcgPipelinedKernel<MT, VT, LEARNED, true>;
+        const void* fn = (const void*)pcgPipelinedKernel<MT, VT, LEARNED>;
         int maxOptin = 0, dev = 0;
         CIPC_CUDA(cudaGetDevice(&dev));
         CIPC_CUDA(cudaDeviceGetAttribute(&maxOptin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -1430,17 +1831,54 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
     }
     a.sliceMax = 0;
     a.rowsPerBlock = 0;
-    const int occ = classic ? 0 : pcgOcc();
-    const void* fn = classic ? (const void*)pcgPersistentKernel<MT, VT, LEARNED>
-                   : occ == 4 ? (const void*)pcgPipelinedKernel<MT, VT, LEARNED, false, 4>
-                   : occ == 3 ? (const void*)pcgPipelinedKernel<MT, VT, LEARNED, false, 3>
-                              : (const void*)pcgPipelinedKernel<MT, VT, LEARNED, false>;
-    int perSM = 0;
-    CIPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, PB, 0));
-    if (perSM < 1) throw std::runtime_error("persistent PCG kernel does not fit on an SM");
-    int grid = std::max(1, std::min(std::min(std::min(perSM, occ >= 3 ? occ : pcgBlocksPerSm()) * smCount, needed), cap));
-    ++g_kernelLaunches;
-    CIPC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(PB), args, 0, c.s));
+    if (classic || sizeof(VT) != sizeof(double)) {
+        const void* fn = (const void*)pcgPersistentKernel<MT, VT, LEARNED>;
+        int perSM = 0;
+        CIPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, PB, 0));
+        if (perSM < 1) throw std::runtime_error("persistent PCG kernel does not fit on an SM");
+        const int grid = std::max(1, std::min(std::min(std::min(perSM, pcgBlocksPerSm()) * smCount, needed), cap));
+        ++g_kernelLaunches;
+        CIPC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(PB), args, 0, c.s));
+        return;
+    }
+    if constexpr (sizeof(VT) == sizeof(double)) {
+        const bool half = LEARNED && !pcgNoPack();
+        if (half) packStream<MT, __half>(c, a.val, true);
+        else packStream<MT, float>(c, a.val, LEARNED);
+        auto view = [](const SellRows& m) { return SellView{m.tile.p, m.col.p, m.val.p}; };
+        a.sA = view(c.sellA); a.sL = view(c.sellL); a.sU = view(c.sellU);
+        // padded gathered vectors
+        const size_t n4 = 4 * (size_t)c.nv;
+        c.pcgGather.reserve(4 * n4);
+        a.g0 = c.pcgGather.p; a.g1 = a.g0 + n4; a.g2 = a.g1 + n4; a.g3 = a.g2 + n4;
+        const int tiles = (c.nv + 7) / 8;
+        const int grid = std::max(1, std::min(std::min(smCount, tiles), cap));
+        a.tilesPerBlock = (tiles + grid - 1) / grid;
+        // the state vectors in shared memory where all eight fit
+        const size_t state = (size_t)a.tilesPerBlock * 24 * sizeof(double) * 8;
+        a.resident = state <= STREAM_STATE_BYTES ? 1 : 0;
+        const size_t smem = a.resident ? state : 0;
+        if (!a.resident) c.pcgState.reserve(8 * (size_t)tiles * 24);
+        a.state = c.pcgState.p;
+        // what every iteration reads: matrix, factor, gathered vectors, diagonal
+        // blocks and the state
+        double bytes = (double)c.sellA.steps * (288 * sizeof(MT) + 128) + c.nv * (2 * 72.0 + 2 * 32.0) + (a.resident ? 0.0 : (double)state * grid);
+        if (LEARNED) bytes += ((double)c.sellL.steps + c.sellU.steps) * (288.0 * (half ? 2 : 4) + 128) + c.nv * 32.0;
+        int dev = 0, l2 = 0;
+        CIPC_CUDA(cudaGetDevice(&dev));
+        CIPC_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+        const bool beyond = bytes > STREAM_L2_SHARE * l2;
+        const void* fn = half ? (beyond ? (const void*)pcgStreamKernel<MT, __half, LEARNED, true> : (const void*)pcgStreamKernel<MT, __half, LEARNED, false>)
+                              : (beyond ? (const void*)pcgStreamKernel<MT, float, LEARNED, true> : (const void*)pcgStreamKernel<MT, float, LEARNED, false>);
+        const int threads = 32 * streamWarps(beyond);
+        CIPC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        int fit = 0;
+        CIPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, threads, smem));
+        if (fit * smCount < grid) throw std::runtime_error("streaming PCG kernel does not fit on an SM");
+        if (debugPcg()) std::fprintf(stderr, "[pcg] streaming launch: %d blocks of %d tiles, state in shared memory %d, beyond L2 %d (%.1f MB)\n", grid, a.tilesPerBlock, a.resident, (int)beyond, bytes * 1e-6);
+        ++g_kernelLaunches;
+        CIPC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem, c.s));
+    }
 }
 
 // Whole PCG in one cooperative launch (grid sized to what is co-resident).
@@ -1465,14 +1903,9 @@ static int runPcgPersistent(Ctx& c, const MT* val, const MT* dval, const VT* b, 
     a.dRowS = dyn ? c.dynRowStart.p : nullptr; a.dRowE = dyn ? c.dynRowEnd.p : nullptr; a.dCol = dyn ? c.dynCol.p : nullptr; a.dVal = dval;
     a.diagExtra = c.diagExtra; a.Dinv = c.Dinv; a.b = b; a.x = x; a.r = r; a.z = z; a.p = p; a.Ap = Ap;
     a.S = nullptr; a.gS = nullptr; a.gD = nullptr; a.t = nullptr;
-    a.gL = a.gU = nullptr; a.gLptr = a.gLcol = a.gUptr = a.gUcol = nullptr;
     if (learned) {
         c.mpT.reserve(3 * (size_t)c.nv);
         a.S = c.mpS.p; a.gS = c.mpGS.p; a.gD = c.mpGD.p; a.t = reinterpret_cast<VT*>(c.mpT.p);
-        if (c.factorPacked) {
-            a.gL = reinterpret_cast<const __half*>(c.gLval.p); a.gU = reinterpret_cast<const __half*>(c.gUval.p);
-            a.gLptr = c.gLptr.p; a.gLcol = c.gLcol.p; a.gUptr = c.gUptr.p; a.gUcol = c.gUcol.p;
-        }
     }
     a.partA = c.red.p; a.partB = c.red.p + PMAX; a.partC = c.red.p + 2 * PMAX;
     // pipelined kernel: six more vectors and two sets of partial sums
@@ -1516,7 +1949,6 @@ static void reservePcg(Ctx& c) {
 // Builds the factor for the current system (network forward, or the exact
 // FSAI); false when block-Jacobi is selected.
 static bool prepareLearned(Ctx& c) {
-    c.factorPacked = false;
     if (c.precond == CIPC_PRECOND_FSAI) {
         mpnnPrepare(c, false);
         fsaiBuild(c);
@@ -1526,12 +1958,6 @@ static bool prepareLearned(Ctx& c) {
         mpnnForward(c);
     } else {
         return false;
-    }
-    // the streaming kernel (systems too large for the single-pass cache)
-    // reads the factor's static part packed by rows in FP16
-    if (!pcgNoPack()) {
-        packFactor(c);
-        c.factorPacked = true;
     }
     return true;
 }

@@ -663,7 +663,7 @@ void cipc_gpu_destroy(cipc_gpu_context* h) {
                                 &c.treeKeys, &c.treeSorted};
         for (auto* d : us) d->free();
         c.sortTmp.free(); c.groundTmp.free(); c.barrierUpper.free(); c.ccdPairs.free(); c.ccdPairCount.free(); c.stepScal.free(); c.faceTree.links.free(); c.edgeTree.links.free();
-        c.gLptr.free(); c.gLcol.free(); c.gLslot.free(); c.gUptr.free(); c.gUcol.free(); c.gUslot.free(); c.gLval.free(); c.gUval.free();
+        c.pcgGather.free(); c.pcgState.free(); c.sellA.free(); c.sellL.free(); c.sellU.free();
         for (DevBvh* t : {&c.faceTree, &c.edgeTree}) {
             t->hashKey.free(); t->hashKeyAlt.free(); t->hashPrim.free(); t->hashPrimAlt.free(); t->hashCount.free(); t->hashOffset.free();
             t->hashBig.free(); t->hashBigFlag.free(); t->hashTmp.free();
@@ -1116,6 +1116,7 @@ extern "C" int cipc_gpu_pcg_bsr(int nv, const int* rowPtr, const int* colIdx, co
         }
         CIPC_CUDA(cudaStreamCreateWithFlags(&c.s, cudaStreamNonBlocking));
         upload(c.rowPtr, rp); upload(c.colIdx, ci); upload(c.diagSlot, diag);
+        c.hRowPtr = rp;
         std::vector<double> v(vals, vals + 9 * (size_t)nnzb);
         if (c.mixed) {
             std::vector<float> f(v.begin(), v.end());
