@@ -54,6 +54,7 @@ template <class T>
 struct DBuf {
     T* p = nullptr;
     size_t cap = 0;
+    bool lent = false;  // p is a piece of a DevSlab
     // grows to twice the request: buffers sized by contact counts grow for a
     // few steps and then stay (a reallocation costs a device-wide wait and
     // page mapping, tens of milliseconds for the pile's contact buffers)
@@ -61,14 +62,40 @@ struct DBuf {
         if (n <= cap) return;
         const bool dbg = debugAlloc();
         const auto t0 = dbg ? std::chrono::steady_clock::now() : std::chrono::steady_clock::time_point();
-        if (p) cudaFree(p);
+        if (p && !lent) cudaFree(p);
+        lent = false;
+        p = nullptr;
         size_t c = n < 64 ? 64 : 2 * n;
         CIPC_CUDA(cudaMalloc(&p, c * sizeof(T)));
         if (dbg) reportAlloc(cap * sizeof(T), c * sizeof(T), std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
         cap = c;
     }
-    void free() { if (p) cudaFree(p); p = nullptr; cap = 0; }
+    void free() { if (p && !lent) cudaFree(p); p = nullptr; cap = 0; lent = false; }
     operator T*() const { return p; }
+};
+
+// One device allocation lent out in 256-byte aligned pieces, for the
+// stand-alone calls: a cudaMalloc or cudaFree takes 150-200 us, and such a call
+// made 28 and 16 of them.  A buffer that outgrows its piece allocates its own.
+struct DevSlab {
+    unsigned char* base = nullptr;
+    size_t used = 0;
+    bool open = false;  // false: pieces are only counted
+    template <class T>
+    void lend(DBuf<T>& d, size_t n) {
+        if (open) { d.p = reinterpret_cast<T*>(base + used); d.cap = n; d.lent = true; }
+        used += (n * sizeof(T) + 255) / 256 * 256;
+    }
+    // plan(slab) lends every piece; it runs once to count and once to lend
+    template <class F>
+    void lendAll(F plan) {
+        plan(*this);
+        CIPC_CUDA(cudaMalloc(&base, used));
+        used = 0;
+        open = true;
+        plan(*this);
+    }
+    ~DevSlab() { if (base) cudaFree(base); }
 };
 
 // Scalars that kernels read (copied to the device once per change).
@@ -108,6 +135,7 @@ struct SellRows {
     DBuf<int> ptr, slot, tile, col;
     DBuf<unsigned char> val;
     int steps = 0;
+    bool laid = false, hasCols = false;  // offsets and columns are in place
     void free() { ptr.free(); slot.free(); tile.free(); col.free(); val.free(); }
 };
 
@@ -320,6 +348,8 @@ void finalizeDynamic(Ctx& c);          // sort + segment dynamic gradient and He
 int pcgSolve(Ctx& c);                  // solves A sol = rhs; returns iterations
 void spmv(Ctx& c, const double* x, double* y);
 void buildRhs(Ctx& c);
+void lendPcg(Ctx& c, DevSlab& slab);   // every buffer of a block-Jacobi solve
+void roundBlocks(Ctx& c, size_t n, const double* src, float* dst);
 
 // ---- reductions (util.cu) ----
 double deviceSum(Ctx& c, const double* v, int n);

@@ -1570,26 +1570,27 @@ __global__ void accdBatchKernel(int n, const int* kind, const double* p, const d
 }  // namespace
 
 void accdBatch(int n, const int* kind, const double* p, const double* d, double eta, double* toi) {
+    DevSlab slab;
     DBuf<int> dk, st;
     DBuf<double> dp, dd, dt;
-    try {
-        dk.reserve(n); dp.reserve(12 * (size_t)n); dd.reserve(12 * (size_t)n); dt.reserve(n); st.reserve(1);
-        CIPC_CUDA(cudaMemcpy(dk.p, kind, sizeof(int) * n, cudaMemcpyHostToDevice));
-        CIPC_CUDA(cudaMemcpy(dp.p, p, sizeof(double) * 12 * (size_t)n, cudaMemcpyHostToDevice));
-        CIPC_CUDA(cudaMemcpy(dd.p, d, sizeof(double) * 12 * (size_t)n, cudaMemcpyHostToDevice));
-        CIPC_CUDA(cudaMemset(st.p, 0, sizeof(int)));
-        launch(accdBatchKernel, blocksFor(n), TB, 0, (cudaStream_t)0, n, (const int*)dk.p, (const double*)dp.p, (const double*)dd.p, eta,
-               dt.p, st.p);
-        CIPC_CUDA(cudaGetLastError());
-        int hs = 0;
-        CIPC_CUDA(cudaMemcpy(toi, dt.p, sizeof(double) * n, cudaMemcpyDeviceToHost));
-        CIPC_CUDA(cudaMemcpy(&hs, st.p, sizeof(int), cudaMemcpyDeviceToHost));
-        if (hs & CIPC_ST_CCD_CAP) throw std::runtime_error("a pair reached the CCD iteration cap");
-    } catch (...) {
-        dk.free(); dp.free(); dd.free(); dt.free(); st.free();
-        throw;
-    }
-    dk.free(); dp.free(); dd.free(); dt.free(); st.free();
+    slab.lendAll([&](DevSlab& s) {
+        s.lend(dp, 12 * (size_t)n);
+        s.lend(dd, 12 * (size_t)n);
+        s.lend(dt, n);
+        s.lend(dk, n);
+        s.lend(st, 1);
+    });
+    CIPC_CUDA(cudaMemcpy(dk.p, kind, sizeof(int) * n, cudaMemcpyHostToDevice));
+    CIPC_CUDA(cudaMemcpy(dp.p, p, sizeof(double) * 12 * (size_t)n, cudaMemcpyHostToDevice));
+    CIPC_CUDA(cudaMemcpy(dd.p, d, sizeof(double) * 12 * (size_t)n, cudaMemcpyHostToDevice));
+    CIPC_CUDA(cudaMemset(st.p, 0, sizeof(int)));
+    launch(accdBatchKernel, blocksFor(n), TB, 0, (cudaStream_t)0, n, (const int*)dk.p, (const double*)dp.p, (const double*)dd.p, eta,
+           dt.p, st.p);
+    CIPC_CUDA(cudaGetLastError());
+    int hs = 0;
+    CIPC_CUDA(cudaMemcpy(toi, dt.p, sizeof(double) * n, cudaMemcpyDeviceToHost));
+    CIPC_CUDA(cudaMemcpy(&hs, st.p, sizeof(int), cudaMemcpyDeviceToHost));
+    if (hs & CIPC_ST_CCD_CAP) throw std::runtime_error("a pair reached the CCD iteration cap");
 }
 
 }  // namespace cipc

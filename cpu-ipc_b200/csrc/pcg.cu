@@ -1607,13 +1607,15 @@ static void tileOffsets(SellRows& m, int nv, const std::vector<int>& ptr) {
         tile[t + 1] = tile[t] + steps;
     }
     m.steps = tile.back();
+    m.laid = true;
     m.tile.reserve(tile.size());
     CIPC_CUDA(cudaMemcpy(m.tile.p, tile.data(), sizeof(int) * tile.size(), cudaMemcpyHostToDevice));
 }
 
 template <class MT, class OT>
 static void packTiles(Ctx& c, SellRows& m, const int* ptr, const int* slotOf, const MT* src) {
-    const bool first = m.col.cap == 0;
+    const bool first = !m.hasCols;
+    m.hasCols = true;
     m.col.reserve(std::max<size_t>((size_t)32 * m.steps, 1));
     m.val.reserve(std::max<size_t>((size_t)288 * sizeof(OT) * m.steps, 16));
     const int nb = std::max(1, std::min(((c.nv + 7) / 8 + VB / 32 - 1) / (VB / 32), 148 * 8));
@@ -1629,10 +1631,10 @@ static void packTiles(Ctx& c, SellRows& m, const int* ptr, const int* slotOf, co
 template <class MT, class FT>
 static void packStream(Ctx& c, const MT* val, bool learned) {
     const int nv = c.nv;
-    if (c.sellA.tile.cap == 0) tileOffsets(c.sellA, nv, c.hRowPtr);
+    if (!c.sellA.laid) tileOffsets(c.sellA, nv, c.hRowPtr);
     packTiles<MT, MT>(c, c.sellA, c.rowPtr, nullptr, val);
     if (!learned) return;
-    if (c.sellL.tile.cap == 0) {
+    if (!c.sellL.laid) {
         std::vector<int> col(c.nnzb);
         CIPC_CUDA(cudaMemcpy(col.data(), c.colIdx.p, sizeof(int) * c.nnzb, cudaMemcpyDeviceToHost));
         std::vector<int> lp(nv + 1, 0), ls, up(nv + 1, 0), us;
@@ -2120,6 +2122,47 @@ static int pcgSolveMixed(Ctx& c) {
     computeDinv(c);
     bool learned = prepareLearned(c);
     return pcgSolveMixed(c, learned);
+}
+
+__global__ void roundBlocksKernel(size_t n, const double* src, float* dst) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) dst[i] = (float)src[i];
+}
+
+void roundBlocks(Ctx& c, size_t n, const double* src, float* dst) {
+    launch(roundBlocksKernel, (int)std::max<size_t>(1, std::min<size_t>((n + VB - 1) / VB, 148 * 8)), VB, 0, c.s, n, src, dst);
+    CIPC_CUDA(cudaGetLastError());
+}
+
+void lendPcg(Ctx& c, DevSlab& slab) {
+    const size_t nv = c.nv, n3 = 3 * nv;
+    for (DBuf<double>* d : {&c.rhs, &c.sol, &c.r, &c.z, &c.p, &c.Ap, &c.corrX, &c.corrR}) slab.lend(*d, n3);
+    slab.lend(c.Dinv, 9 * nv);
+    slab.lend(c.red, 4 * PMAX + 16);
+    slab.lend(c.scal, 16);
+    slab.lend(c.counters, 16);
+    slab.lend(c.rF, n3);
+    if (c.mixed)
+        for (DBuf<float>* d : {&c.zF, &c.pF, &c.ApF, &c.xF, &c.DinvF}) slab.lend(*d, n3);
+    slab.lend(c.pcgPipe, 6 * n3 + 6);
+    slab.lend(c.pcgParts, 6 * (size_t)PIPE_PMAX);
+    slab.lend(c.pcgBar, BAR_WORDS);
+    int dev = 0, sms = 0;
+    CIPC_CUDA(cudaGetDevice(&dev));
+    CIPC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (nv > (size_t)sms * ROWS_PER_BLOCK) {
+        // more rows than the single-pass launch can hold: the tiles too
+        const size_t tiles = (nv + 7) / 8;
+        if (!c.sellA.steps)
+            for (size_t t = 0; t < tiles; ++t) {
+                int most = 0;
+                for (size_t r = 8 * t; r < std::min(nv, 8 * t + 8); ++r) most = std::max(most, c.hRowPtr[r + 1] - c.hRowPtr[r]);
+                c.sellA.steps += (most + GROUP - 1) / GROUP;
+            }
+        slab.lend(c.sellA.tile, tiles + 1);
+        slab.lend(c.sellA.col, 32 * (size_t)c.sellA.steps);
+        slab.lend(c.sellA.val, 288 * (c.mixed ? sizeof(float) : sizeof(double)) * (size_t)c.sellA.steps);
+        slab.lend(c.pcgGather, 16 * nv);
+    }
 }
 
 int pcgSolve(Ctx& c) { return c.mixed ? pcgSolveMixed(c) : pcgSolve64(c); }

@@ -1093,6 +1093,21 @@ extern "C" int cipc_gpu_pcg_bsr(int nv, const int* rowPtr, const int* colIdx, co
     };
     if (nv <= 0 || !rowPtr || !colIdx || !vals || !rhs || !sol) return fail("invalid arguments", CIPC_ERR_INVALID_ARGUMENT);
     Ctx c;
+    DevSlab slab;  // freed last
+    struct Release {
+        Ctx& c;
+        ~Release() {
+            if (c.s) cudaStreamSynchronize(c.s);
+            for (DBuf<double>* d : {&c.valD, &c.diagExtra, &c.rhs, &c.sol, &c.r, &c.z, &c.p, &c.Ap, &c.Dinv, &c.red, &c.scal, &c.corrX, &c.corrR, &c.pcgPipe,
+                                    &c.pcgParts, &c.pcgGather, &c.pcgState, &c.scratch, &c.sums, &c.energyBuf})
+                d->free();
+            for (DBuf<float>* d : {&c.valF, &c.rF, &c.zF, &c.pF, &c.ApF, &c.xF, &c.DinvF}) d->free();
+            for (DBuf<int>* d : {&c.rowPtr, &c.colIdx, &c.diagSlot, &c.counters, &c.status}) d->free();
+            c.pcgBar.free();
+            c.sellA.free();
+            if (c.s) cudaStreamDestroy(c.s);
+        }
+    } release{c};
     try {
         c.nv = nv;
         if (options) {
@@ -1103,44 +1118,47 @@ extern "C" int cipc_gpu_pcg_bsr(int nv, const int* rowPtr, const int* colIdx, co
         int nnzb = rowPtr[nv];
         if (nnzb < 0 || rowPtr[0] < 0) return fail("row pointers must be non-negative and non-decreasing", CIPC_ERR_INVALID_ARGUMENT);
         c.nnzb = nnzb;
-        std::vector<int> rp(rowPtr, rowPtr + nv + 1), ci(colIdx, colIdx + nnzb), diag(nv, -1);
+        c.hRowPtr.assign(rowPtr, rowPtr + nv + 1);
+        std::vector<int> diag(nv, -1);
         for (int r = 0; r < nv; ++r) {
-            if (rp[r] < 0 || rp[r + 1] < rp[r]) return fail("row pointers must be non-negative and non-decreasing", CIPC_ERR_INVALID_ARGUMENT);
+            if (rowPtr[r] < 0 || rowPtr[r + 1] < rowPtr[r]) return fail("row pointers must be non-negative and non-decreasing", CIPC_ERR_INVALID_ARGUMENT);
+            if (rowPtr[r + 1] > nnzb) return fail("row pointers must be non-negative and non-decreasing", CIPC_ERR_INVALID_ARGUMENT);
             int nd = 0;
-            for (int k = rp[r]; k < rp[r + 1]; ++k) {
-                if (ci[k] < 0 || ci[k] >= nv) return fail("column index out of range", CIPC_ERR_INVALID_ARGUMENT);
-                if (ci[k] == r) { diag[r] = k; ++nd; }
+            for (int k = rowPtr[r]; k < rowPtr[r + 1]; ++k) {
+                if (colIdx[k] < 0 || colIdx[k] >= nv) return fail("column index out of range", CIPC_ERR_INVALID_ARGUMENT);
+                if (colIdx[k] == r) { diag[r] = k; ++nd; }
             }
             // the block-Jacobi inverse needs the row's one diagonal block
             if (nd != 1) return fail("every block row needs exactly one diagonal block", CIPC_ERR_INVALID_ARGUMENT);
         }
         CIPC_CUDA(cudaStreamCreateWithFlags(&c.s, cudaStreamNonBlocking));
-        upload(c.rowPtr, rp); upload(c.colIdx, ci); upload(c.diagSlot, diag);
-        c.hRowPtr = rp;
-        std::vector<double> v(vals, vals + 9 * (size_t)nnzb);
-        if (c.mixed) {
-            std::vector<float> f(v.begin(), v.end());
-            upload(c.valF, f);
-        } else {
-            upload(c.valD, v);
-        }
-        upload(c.diagExtra, std::vector<double>(9 * (size_t)nv, 0.0));
-        upload(c.rhs, std::vector<double>(rhs, rhs + 3 * (size_t)nv));
-        c.counters.reserve(16);
-        c.status.reserve(4);
+        const size_t nval = 9 * (size_t)nnzb;
+        slab.lendAll([&](DevSlab& s) {
+            s.lend(c.rowPtr, nv + 1);
+            s.lend(c.colIdx, nnzb);
+            s.lend(c.diagSlot, nv);
+            s.lend(c.valD, nval);
+            if (c.mixed) s.lend(c.valF, nval);
+            s.lend(c.diagExtra, 9 * (size_t)nv);
+            s.lend(c.status, 4);
+            lendPcg(c, s);
+        });
+        upload(c.rowPtr, c.hRowPtr);
+        upload(c.diagSlot, diag);
+        CIPC_CUDA(cudaMemcpy(c.colIdx.p, colIdx, sizeof(int) * (size_t)nnzb, cudaMemcpyHostToDevice));
+        CIPC_CUDA(cudaMemcpy(c.valD.p, vals, sizeof(double) * nval, cudaMemcpyHostToDevice));
+        CIPC_CUDA(cudaMemcpy(c.rhs.p, rhs, sizeof(double) * 3 * (size_t)nv, cudaMemcpyHostToDevice));
+        CIPC_CUDA(cudaMemsetAsync(c.diagExtra.p, 0, sizeof(double) * 9 * (size_t)nv, c.s));
+        // pageable copies return when the data is staged, not when it has arrived
+        CIPC_CUDA(cudaStreamSynchronize((cudaStream_t)0));
+        if (c.mixed) roundBlocks(c, nval, c.valD, c.valF);
         int it = pcgSolve(c);
         CIPC_CUDA(cudaMemcpy(sol, c.sol.p, sizeof(double) * 3 * nv, cudaMemcpyDeviceToHost));
         if (iterations) *iterations = it;
         if (relResidual) *relResidual = c.lastPcgRelRes;
     } catch (const std::exception& e) {
-        int code = std::string(e.what()).find("did not converge") != std::string::npos ? CIPC_ERR_NOT_CONVERGED : CIPC_ERR_CUDA;
-        c.rowPtr.free(); c.colIdx.free(); c.diagSlot.free(); c.valD.free(); c.valF.free(); c.diagExtra.free(); c.rhs.free();
-        c.sol.free(); c.r.free(); c.z.free(); c.p.free(); c.Ap.free(); c.Dinv.free(); c.red.free(); c.scal.free(); c.counters.free(); c.status.free();
-        if (c.s) cudaStreamDestroy(c.s);
+        const int code = std::string(e.what()).find("did not converge") != std::string::npos ? CIPC_ERR_NOT_CONVERGED : CIPC_ERR_CUDA;
         return fail(e.what(), code);
     }
-    c.rowPtr.free(); c.colIdx.free(); c.diagSlot.free(); c.valD.free(); c.valF.free(); c.diagExtra.free(); c.rhs.free();
-    c.sol.free(); c.r.free(); c.z.free(); c.p.free(); c.Ap.free(); c.Dinv.free(); c.red.free(); c.scal.free(); c.counters.free(); c.status.free();
-    if (c.s) cudaStreamDestroy(c.s);
     return CIPC_OK;
 }
