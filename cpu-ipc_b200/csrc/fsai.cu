@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(32 * FS_WARPS) fsaiKernel(int nv, const int* r
         // is subtracted from the rows that remain, n steps in a chain.  With one
         // lane per right-hand side (n^2 steps), a lane per row in the Cholesky
         // updates and a full square in shared memory a Newton system of the
-        // 128-vertex cloth drape (17,715 rows) took 3.13 ms on a B200, now 2.84.
+        // 128-vertex cloth drape (17,715 rows) took 3.05 ms on a B200, now 2.84.
         {
             double s[FS_ROWS][3];
 #pragma unroll

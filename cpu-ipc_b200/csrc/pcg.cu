@@ -709,6 +709,12 @@ __global__ void __launch_bounds__(PB) pcgPersistentKernel(PcgArgs<MT, VT> a) {
 // iteration then reads the matrix rows from shared memory and only the
 // gathered vectors from L2.
 constexpr int ROWS_PER_BLOCK = PB / GROUP;
+// Rows per block of a small system: fewer and fuller blocks make the grid
+// barrier and its sums cheaper.  Measured per solve on a B200 with at least 3 (one
+// block per SM), 16, 32 and 64 rows: 432 rows 2.78, 2.63, 2.62, 2.58 ms; 1,881
+// rows (13 a block) 0.29, 0.30, 0.27, 0.26 ms; 1,458 FP32 rows 4.55, 4.33, 4.38,
+// 4.19 ms.
+constexpr int SINGLE_MIN_ROWS = 64;
 constexpr int STATE_VECS = 9;  // x r u w z q s p, and the row's own m
 
 struct SmemLayout {
@@ -1799,8 +1805,9 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
         // solve and stages them in shared memory.  The largest configuration
         // that keeps every block resident is taken: the factor's blocks
         // cached or not, a contact window of 512 down to 0 slots.
-        // rows spread evenly over at least one block per SM
-        const int rows = (c.nv + std::max(needed, smCount) - 1) / std::max(needed, smCount);
+        // rows spread evenly over one block per SM or more, SINGLE_MIN_ROWS at least
+        const int rows = std::max(SINGLE_MIN_ROWS, (c.nv + std::max(needed, smCount) - 1) / std::max(needed, smCount));
+        const int threads = std::min(PB, (rows * GROUP + 31) / 32 * 32);
         const int nbRows = (c.nv + rows - 1) / rows;
         a.rowsPerBlock = rows;
         a.sliceMax = pcgSliceMax(c, rows);
@@ -1817,7 +1824,7 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
                 if (smem + 4096 > (size_t)maxOptin) continue;
                 CIPC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 int perSM = 0;
-                CIPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, PB, smem));
+                CIPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, threads, smem));
                 if (perSM >= 1 && nbRows <= perSM * smCount && nbRows <= cap) {
                     a.dynCap = dc;
                     a.cacheG = cg;
@@ -1825,7 +1832,7 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
                         std::fprintf(stderr, "[pcg] single-pass launch: %d blocks of %d rows, slice %d, contact window %d, factor cached %d, %zu B shared\n",
                                      nbRows, rows, a.sliceMax, dc, cg, smem);
                     ++g_kernelLaunches;
-                    CIPC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(nbRows), dim3(PB), args, smem, c.s));
+                    CIPC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(nbRows), dim3(threads), args, smem, c.s));
                     return;
                 }
             }
