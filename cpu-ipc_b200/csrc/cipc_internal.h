@@ -307,6 +307,21 @@ inline void hostSync(Ctx& c) {
     CIPC_CUDA(cudaStreamSynchronize(c.s));
 }
 
+// A host array into a buffer of the context, on the context's stream, where the
+// kernels that read it follow: that stream does not wait for the legacy one, on
+// which a copy from pageable memory may return before the data has arrived.
+// The array may go when this returns.
+inline void copyIn(Ctx& c, void* dst, const void* src, size_t bytes) {
+    if (!bytes) return;
+    CIPC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c.s));
+    hostSync(c);
+}
+template <class T>
+void upload(Ctx& c, DBuf<T>& d, const std::vector<T>& h) {
+    d.reserve(h.empty() ? 1 : h.size());
+    copyIn(c, d.p, h.data(), h.size() * sizeof(T));
+}
+
 void buildStaticPattern(Ctx& c, const std::vector<int>& tets, const std::vector<int>& tris, const std::vector<int>& bendV);
 void assembleElastic(Ctx& c);          // vtxGrad, diagExtra, element blocks, static BSR values, element gradient
 void tetGradient(Ctx& c);              // elemG of the tetrahedra only (no Hessian)

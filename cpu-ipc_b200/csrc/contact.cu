@@ -928,12 +928,12 @@ void closeConstraintRecord(Ctx& c) {
     c.closeG.reserve(std::max(c.nCloseG, 1)); c.closeGVal.reserve(std::max(c.nCloseG, 1));
     c.closeS.reserve(4 * std::max(c.nCloseS, 1)); c.closeSVal.reserve(std::max(c.nCloseS, 1));
     if (c.nCloseG) {
-        CIPC_CUDA(cudaMemcpy(c.closeG.p, cg.data(), cg.size() * sizeof(int), cudaMemcpyHostToDevice));
-        CIPC_CUDA(cudaMemcpy(c.closeGVal.p, cgv.data(), cgv.size() * sizeof(double), cudaMemcpyHostToDevice));
+        copyIn(c, c.closeG.p, cg.data(), cg.size() * sizeof(int));
+        copyIn(c, c.closeGVal.p, cgv.data(), cgv.size() * sizeof(double));
     }
     if (c.nCloseS) {
-        CIPC_CUDA(cudaMemcpy(c.closeS.p, cs.data(), cs.size() * sizeof(int), cudaMemcpyHostToDevice));
-        CIPC_CUDA(cudaMemcpy(c.closeSVal.p, csv.data(), csv.size() * sizeof(double), cudaMemcpyHostToDevice));
+        copyIn(c, c.closeS.p, cs.data(), cs.size() * sizeof(int));
+        copyIn(c, c.closeSVal.p, csv.data(), csv.size() * sizeof(double));
     }
 }
 

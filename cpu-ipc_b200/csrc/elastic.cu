@@ -597,13 +597,9 @@ void buildStaticPattern(Ctx& c, const std::vector<int>& tets, const std::vector<
     std::vector<int> gcPtr(nv + 1, 0), gcIdx(gc.size());
     for (size_t k = 0; k < gc.size(); ++k) { gcPtr[gc[k].first + 1]++; gcIdx[k] = gc[k].second; }
     for (int v = 0; v < nv; ++v) gcPtr[v + 1] += gcPtr[v];
-    auto up = [&](DBuf<int>& d, const std::vector<int>& h) {
-        d.reserve(std::max<size_t>(h.size(), 1));
-        if (!h.empty()) CIPC_CUDA(cudaMemcpy(d.p, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice));
-    };
-    up(c.rowPtr, rowPtr); up(c.colIdx, col); up(c.diagSlot, diag); up(c.hcPtr, hcPtr); up(c.hcIdx, hcIdx);
+    upload(c, c.rowPtr, rowPtr); upload(c, c.colIdx, col); upload(c, c.diagSlot, diag); upload(c, c.hcPtr, hcPtr); upload(c, c.hcIdx, hcIdx);
     c.hRowPtr = rowPtr;
-    up(c.gcPtr, gcPtr); up(c.gcIdx, gcIdx);
+    upload(c, c.gcPtr, gcPtr); upload(c, c.gcIdx, gcIdx);
     c.valD.reserve((size_t)9 * c.nnzb);
     c.valF.reserve((size_t)9 * c.nnzb);
     c.elemG.reserve((size_t)3 * std::max(1, c.nElemGrad));

@@ -1605,7 +1605,7 @@ __global__ void packTilesKernel(int nv, const int* ptr, const int* slotOf, const
 }
 
 // Step offsets of the tiles of 8 rows with the given row offsets.
-static void tileOffsets(SellRows& m, int nv, const std::vector<int>& ptr) {
+static void tileOffsets(Ctx& c, SellRows& m, int nv, const std::vector<int>& ptr) {
     std::vector<int> tile((nv + 7) / 8 + 1, 0);
     for (int t = 0; 8 * t < nv; ++t) {
         int steps = 0;
@@ -1614,8 +1614,7 @@ static void tileOffsets(SellRows& m, int nv, const std::vector<int>& ptr) {
     }
     m.steps = tile.back();
     m.laid = true;
-    m.tile.reserve(tile.size());
-    CIPC_CUDA(cudaMemcpy(m.tile.p, tile.data(), sizeof(int) * tile.size(), cudaMemcpyHostToDevice));
+    upload(c, m.tile, tile);
 }
 
 template <class MT, class OT>
@@ -1637,7 +1636,7 @@ static void packTiles(Ctx& c, SellRows& m, const int* ptr, const int* slotOf, co
 template <class MT, class FT>
 static void packStream(Ctx& c, const MT* val, bool learned) {
     const int nv = c.nv;
-    if (!c.sellA.laid) tileOffsets(c.sellA, nv, c.hRowPtr);
+    if (!c.sellA.laid) tileOffsets(c, c.sellA, nv, c.hRowPtr);
     packTiles<MT, MT>(c, c.sellA, c.rowPtr, nullptr, val);
     if (!learned) return;
     if (!c.sellL.laid) {
@@ -1653,13 +1652,9 @@ static void packStream(Ctx& c, const MT* val, bool learned) {
             lp[r + 1] = (int)ls.size();
             up[r + 1] = (int)us.size();
         }
-        auto up_ = [&](DBuf<int>& d, const std::vector<int>& h) {
-            d.reserve(std::max<size_t>(h.size(), 1));
-            if (!h.empty()) CIPC_CUDA(cudaMemcpy(d.p, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice));
-        };
-        up_(c.sellL.ptr, lp); up_(c.sellL.slot, ls); up_(c.sellU.ptr, up); up_(c.sellU.slot, us);
-        tileOffsets(c.sellU, nv, up);
-        tileOffsets(c.sellL, nv, lp);
+        upload(c, c.sellL.ptr, lp); upload(c, c.sellL.slot, ls); upload(c, c.sellU.ptr, up); upload(c, c.sellU.slot, us);
+        tileOffsets(c, c.sellU, nv, up);
+        tileOffsets(c, c.sellL, nv, lp);
     }
     packTiles<float, FT>(c, c.sellL, c.sellL.ptr, c.sellL.slot, (const float*)c.mpGS);
     packTiles<float, FT>(c, c.sellU, c.sellU.ptr, c.sellU.slot, (const float*)c.mpGS);

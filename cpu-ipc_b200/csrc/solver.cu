@@ -455,12 +455,6 @@ void solveIPCStep(Ctx& c, cipc_step_stats& st) {
     c.stepIndex++;
 }
 
-template <class T>
-void upload(DBuf<T>& d, const std::vector<T>& h) {
-    d.reserve(std::max<size_t>(h.size(), 1));
-    if (!h.empty()) CIPC_CUDA(cudaMemcpy(d.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
-}
-
 Ctx* createContext(const cipc_scene_desc* s, const cipc_linear_options* o) {
     if (!s || s->nv <= 0 || !s->x || !s->btype) throw InvalidArgument("scene needs vertices and boundary types");
     if (s->nt < 0 || s->nf < 0 || (s->nt > 0 && !s->tets) || (s->nf > 0 && !s->tris)) throw InvalidArgument("invalid element arrays");
@@ -537,27 +531,27 @@ Ctx* createContext(const cipc_scene_desc* s, const cipc_linear_options* o) {
         for (int v : c->hDirIdx) if (v < 0 || v >= s->nv || c->hBtype[v] == 0) throw InvalidArgument("animated Dirichlet vertices must be marked constrained");
         CIPC_CUDA(cudaStreamCreateWithFlags(&c->s, cudaStreamNonBlocking));
         size_t n3 = 3 * (size_t)s->nv;
-        upload(c->x, in.x); upload(c->rest, in.x); upload(c->vp, in.x);
+        upload(*c, c->x, in.x); upload(*c, c->rest, in.x); upload(*c, c->vp, in.x);
         c->x0.reserve(n3); c->xt.reserve(n3); c->dir.reserve(n3); c->grad.reserve(n3);
         std::vector<double> vel(n3, 0.0);
         if (s->vel) vel.assign(s->vel, s->vel + n3);
-        upload(c->vel, vel);
-        upload(c->mass, r.mass);
-        upload(c->btype, c->hBtype);
-        upload(c->tets, in.tets); upload(c->tris, in.tris);
-        upload(c->DmInv, r.DmInv); upload(c->vol, r.vol); upload(c->tetMu, r.tetMu); upload(c->tetLam, r.tetLam);
-        upload(c->DmInv2, r.DmInv2); upload(c->area, r.area);
-        upload(c->bendV, r.bendV); upload(c->bendQ, r.bendQ);
+        upload(*c, c->vel, vel);
+        upload(*c, c->mass, r.mass);
+        upload(*c, c->btype, c->hBtype);
+        upload(*c, c->tets, in.tets); upload(*c, c->tris, in.tris);
+        upload(*c, c->DmInv, r.DmInv); upload(*c, c->vol, r.vol); upload(*c, c->tetMu, r.tetMu); upload(*c, c->tetLam, r.tetLam);
+        upload(*c, c->DmInv2, r.DmInv2); upload(*c, c->area, r.area);
+        upload(*c, c->bendV, r.bendV); upload(*c, c->bendQ, r.bendQ);
         c->hinge = in.hingeBending ? 1 : 0;
-        if (c->hinge) { upload(c->hingeW, r.hingeW); upload(c->hingeTh0, r.hingeTh0); }
-        upload(c->faces, r.faces); upload(c->surfVerts, r.surfVerts); upload(c->edges, r.edges);
-        upload(c->softIdx, c->hSoftIdx);
+        if (c->hinge) { upload(*c, c->hingeW, r.hingeW); upload(*c, c->hingeTh0, r.hingeTh0); }
+        upload(*c, c->faces, r.faces); upload(*c, c->surfVerts, r.surfVerts); upload(*c, c->edges, r.edges);
+        upload(*c, c->softIdx, c->hSoftIdx);
         std::vector<double> tgt;
         for (int v : c->hSoftIdx) for (int q = 0; q < 3; ++q) tgt.push_back(in.x[3 * v + q]);
-        upload(c->softTarget, tgt);
-        upload(c->dirIdx, c->hDirIdx);
+        upload(*c, c->softTarget, tgt);
+        upload(*c, c->dirIdx, c->hDirIdx);
         c->status.reserve(4);
-        CIPC_CUDA(cudaMemset(c->status.p, 0, sizeof(int)));
+        CIPC_CUDA(cudaMemsetAsync(c->status.p, 0, sizeof(int), c->s));
         c->counters.reserve(16);
         c->scratch.reserve(2048);
         buildStaticPattern(*c, in.tets, in.tris, r.bendV);
@@ -704,8 +698,7 @@ int cipc_gpu_set_state(cipc_gpu_context* h, int which, const double* in) {
     return guarded(h, [&](Ctx& c) {
         if (!in) throw InvalidArgument("null input");
         if (which == 4) throw InvalidArgument("rest positions are fixed at creation");
-        hostSync(c);
-        CIPC_CUDA(cudaMemcpy(stateBuf(c, which)->p, in, sizeof(double) * 3 * c.nv, cudaMemcpyHostToDevice));
+        copyIn(c, stateBuf(c, which)->p, in, sizeof(double) * 3 * c.nv);
     });
 }
 
@@ -860,7 +853,7 @@ int cipc_gpu_energy(cipc_gpu_context* h, double kappa, double* e) {
 
 int cipc_gpu_step_bounds(cipc_gpu_context* h, const double* dir, double alphaIn, double* out) {
     return guarded(h, [&](Ctx& c) {
-        CIPC_CUDA(cudaMemcpy(c.dir.p, dir, sizeof(double) * 3 * c.nv, cudaMemcpyHostToDevice));
+        copyIn(c, c.dir.p, dir, sizeof(double) * 3 * c.nv);
         out[0] = std::min(1.0, groundStepBound(c));
         out[1] = partialCCD(c, alphaIn);
         out[2] = cflBound(c);
@@ -1143,14 +1136,12 @@ extern "C" int cipc_gpu_pcg_bsr(int nv, const int* rowPtr, const int* colIdx, co
             s.lend(c.status, 4);
             lendPcg(c, s);
         });
-        upload(c.rowPtr, c.hRowPtr);
-        upload(c.diagSlot, diag);
-        CIPC_CUDA(cudaMemcpy(c.colIdx.p, colIdx, sizeof(int) * (size_t)nnzb, cudaMemcpyHostToDevice));
-        CIPC_CUDA(cudaMemcpy(c.valD.p, vals, sizeof(double) * nval, cudaMemcpyHostToDevice));
-        CIPC_CUDA(cudaMemcpy(c.rhs.p, rhs, sizeof(double) * 3 * (size_t)nv, cudaMemcpyHostToDevice));
+        upload(c, c.rowPtr, c.hRowPtr);
+        upload(c, c.diagSlot, diag);
+        copyIn(c, c.colIdx.p, colIdx, sizeof(int) * (size_t)nnzb);
+        copyIn(c, c.valD.p, vals, sizeof(double) * nval);
+        copyIn(c, c.rhs.p, rhs, sizeof(double) * 3 * (size_t)nv);
         CIPC_CUDA(cudaMemsetAsync(c.diagExtra.p, 0, sizeof(double) * 9 * (size_t)nv, c.s));
-        // pageable copies return when the data is staged, not when it has arrived
-        CIPC_CUDA(cudaStreamSynchronize((cudaStream_t)0));
         if (c.mixed) roundBlocks(c, nval, c.valD, c.valF);
         int it = pcgSolve(c);
         CIPC_CUDA(cudaMemcpy(sol, c.sol.p, sizeof(double) * 3 * nv, cudaMemcpyDeviceToHost));
