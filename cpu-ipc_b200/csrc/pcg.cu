@@ -1788,6 +1788,18 @@ static int pcgSliceMax(Ctx& c, int rows) {
     return c.pcgSliceMax;
 }
 
+// Lets a kernel ask for as much dynamic shared memory as a block can have.  The
+// limit belongs to the process, not to the launch: a limit of one system's size
+// would be lowered by another thread's smaller system between here and the launch.
+static void allowSharedMemory(const void* fn) {
+    int dev = 0, optin = 0;
+    CIPC_CUDA(cudaGetDevice(&dev));
+    CIPC_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    cudaFuncAttributes fa;
+    CIPC_CUDA(cudaFuncGetAttributes(&fa, fn));
+    CIPC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+}
+
 template <class MT, class VT, bool LEARNED>
 static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool classic) {
     int needed = std::max(1, (c.nv * GROUP + PB - 1) / PB);
@@ -1810,6 +1822,7 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
         int maxOptin = 0, dev = 0;
         CIPC_CUDA(cudaGetDevice(&dev));
         CIPC_CUDA(cudaDeviceGetAttribute(&maxOptin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        allowSharedMemory(fn);
         const bool dyn = a.dRowS != nullptr;
         static const int dynCaps[] = {512, 256, 128, 0};
         for (int cg = LEARNED ? 1 : 0; cg >= 0; --cg) {
@@ -1817,7 +1830,6 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
                 if (!dyn && dc > 0) continue;
                 size_t smem = smemLayout(a.sliceMax, dc, cg != 0, (int)sizeof(MT), (int)sizeof(VT)).total;
                 if (smem + 4096 > (size_t)maxOptin) continue;
-                CIPC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 int perSM = 0;
                 CIPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, threads, smem));
                 if (perSM >= 1 && nbRows <= perSM * smCount && nbRows <= cap) {
@@ -1875,7 +1887,7 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
         const void* fn = half ? (beyond ? (const void*)pcgStreamKernel<MT, __half, LEARNED, true> : (const void*)pcgStreamKernel<MT, __half, LEARNED, false>)
                               : (beyond ? (const void*)pcgStreamKernel<MT, float, LEARNED, true> : (const void*)pcgStreamKernel<MT, float, LEARNED, false>);
         const int threads = 32 * streamWarps(beyond);
-        CIPC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allowSharedMemory(fn);
         int fit = 0;
         CIPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, threads, smem));
         if (fit * smCount < grid) throw std::runtime_error("streaming PCG kernel does not fit on an SM");
