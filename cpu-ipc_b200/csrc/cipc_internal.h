@@ -65,9 +65,11 @@ struct DBuf {
         if (p && !lent) cudaFree(p);
         lent = false;
         p = nullptr;
+        const size_t old = cap;
+        cap = 0;  // until the allocation has succeeded
         size_t c = n < 64 ? 64 : 2 * n;
         CIPC_CUDA(cudaMalloc(&p, c * sizeof(T)));
-        if (dbg) reportAlloc(cap * sizeof(T), c * sizeof(T), std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
+        if (dbg) reportAlloc(old * sizeof(T), c * sizeof(T), std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
         cap = c;
     }
     void free() { if (p && !lent) cudaFree(p); p = nullptr; cap = 0; lent = false; }

@@ -38,9 +38,11 @@ class FakeRuntime:
 def _library():
     lib_build.build()
     objs = [os.path.join(lib_build.OUT, n + ".o") for n in list(lib_build.UNITS) + list(lib_build.HOST_UNITS)]
-    so = os.path.join(tempfile.mkdtemp(), "libcipc_fake_runtime.so")
+    tmp = tempfile.mkdtemp()
+    so, harness = os.path.join(tmp, "libcipc_fake_runtime.so"), os.path.join(tmp, "device_buffer_harness.o")
+    subprocess.run([lib_build.NVCC, *lib_build.ARCH, *lib_build.COMMON, "-c", os.path.join(HERE, "device_buffer_harness.cu"), "-o", harness], check=True)
     subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-Wl,-z,defs", "-I/usr/local/cuda/include",
-                    os.path.join(HERE, "fake_cudart.cpp"), *objs, "-o", so, "-lpthread", "-ldl", "-lrt"], check=True)
+                    os.path.join(HERE, "fake_cudart.cpp"), harness, *objs, "-o", so, "-lpthread", "-ldl", "-lrt"], check=True)
     return so
 
 
