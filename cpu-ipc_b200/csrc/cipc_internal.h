@@ -11,11 +11,15 @@
 #include <string>
 #include <vector>
 
+// Throws on an error, which it takes out of the runtime's record: the checks of
+// later launches would report it again.
 #define CIPC_CUDA(call)                                                                          \
     do {                                                                                         \
         cudaError_t e__ = (call);                                                                \
-        if (e__ != cudaSuccess)                                                                  \
+        if (e__ != cudaSuccess) {                                                                \
+            cudaGetLastError();                                                                  \
             throw cipc::CudaError(std::string(#call) + ": " + cudaGetErrorString(e__));          \
+        }                                                                                        \
     } while (0)
 
 namespace cipc {

@@ -4,7 +4,8 @@
 
 extern "C" void fake_fail_malloc(int nth);
 
-// 1 where a buffer whose growth failed is whole again after a smaller request
+// 1 where a buffer whose growth failed is whole again after a smaller request,
+// and a launch after that would not be taken for failed
 extern "C" int buffer_recovers(int first, int failing, int again) {
     cipc::DBuf<double> d;
     d.reserve(first);
@@ -17,7 +18,7 @@ extern "C" int buffer_recovers(int first, int failing, int again) {
     }
     fake_fail_malloc(0);
     d.reserve(again);
-    const bool whole = failed && d.p && d.cap >= (size_t)again;
+    const bool whole = failed && d.p && d.cap >= (size_t)again && cudaPeekAtLastError() == cudaSuccess;
     d.free();
     return whole;
 }
