@@ -1613,20 +1613,20 @@ static void tileOffsets(Ctx& c, SellRows& m, int nv, const std::vector<int>& ptr
         tile[t + 1] = tile[t] + steps;
     }
     m.steps = tile.back();
-    m.laid = true;
     upload(c, m.tile, tile);
+    m.laid = true;
 }
 
 template <class MT, class OT>
 static void packTiles(Ctx& c, SellRows& m, const int* ptr, const int* slotOf, const MT* src) {
     const bool first = !m.hasCols;
-    m.hasCols = true;
     m.col.reserve(std::max<size_t>((size_t)32 * m.steps, 1));
     m.val.reserve(std::max<size_t>((size_t)288 * sizeof(OT) * m.steps, 16));
     const int nb = std::max(1, std::min(((c.nv + 7) / 8 + VB / 32 - 1) / (VB / 32), 148 * 8));
     launch(packTilesKernel<MT, OT>, nb, VB, 0, c.s, c.nv, ptr, slotOf, (const int*)c.colIdx, src, (const int*)m.tile, first ? m.col.p : (int*)nullptr,
            reinterpret_cast<OT*>(m.val.p));
     CIPC_CUDA(cudaGetLastError());
+    m.hasCols = true;
 }
 
 // The static matrix and, with a factor, its static blocks in tiles: per row
