@@ -1808,16 +1808,16 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
     a.dynCap = 0;
     a.cacheG = 0;
     if (!classic && !pcgNoCache() && !c.hRowPtr.empty() && needed <= cap) {
-        // single-pass launch: each block owns ROWS_PER_BLOCK rows for the whole
-        // solve and stages them in shared memory.  The largest configuration
-        // that keeps every block resident is taken: the factor's blocks
-        // cached or not, a contact window of 512 down to 0 slots.
-        // rows spread evenly over one block per SM or more, SINGLE_MIN_ROWS at least
-        const int rows = std::max(SINGLE_MIN_ROWS, (c.nv + std::max(needed, smCount) - 1) / std::max(needed, smCount));
-        const int threads = std::min(PB, (rows * GROUP + 31) / 32 * 32);
-        const int nbRows = (c.nv + rows - 1) / rows;
-        a.rowsPerBlock = rows;
-        a.sliceMax = pcgSliceMax(c, rows);
+        // single-pass launch: each block owns its rows for the whole solve and
+        // stages them in shared memory.  The largest configuration that keeps
+        // every block resident is taken: the factor's blocks cached or not, a
+        // contact window of 512 down to 0 slots.  Rows are spread evenly over one
+        // block per SM or more, SINGLE_MIN_ROWS at least.  Where so many wide rows
+        // do not fit, the streaming kernel takes a block-Jacobi solve as fast (443
+        // rows of 161 blocks on a B200: 0.59 ms with 8 rows a block, 0.58 streamed;
+        // FP32 0.74 and 0.51); a factor, which it would round to FP16, stays here
+        // with fewer rows a block, down to the even spread.
+        const int even = (c.nv + std::max(needed, smCount) - 1) / std::max(needed, smCount);
         const void* fn = (const void*)pcgPipelinedKernel<MT, VT, LEARNED>;
         int maxOptin = 0, dev = 0;
         CIPC_CUDA(cudaGetDevice(&dev));
@@ -1826,21 +1826,28 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
         const bool dyn = a.dRowS != nullptr;
         static const int dynCaps[] = {512, 256, 128, 0};
         for (int cg = LEARNED ? 1 : 0; cg >= 0; --cg) {
-            for (int dc : dynCaps) {
-                if (!dyn && dc > 0) continue;
-                size_t smem = smemLayout(a.sliceMax, dc, cg != 0, (int)sizeof(MT), (int)sizeof(VT)).total;
-                if (smem + 4096 > (size_t)maxOptin) continue;
-                int perSM = 0;
-                CIPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, threads, smem));
-                if (perSM >= 1 && nbRows <= perSM * smCount && nbRows <= cap) {
-                    a.dynCap = dc;
-                    a.cacheG = cg;
-                    if (debugPcg())
-                        std::fprintf(stderr, "[pcg] single-pass launch: %d blocks of %d rows, slice %d, contact window %d, factor cached %d, %zu B shared\n",
-                                     nbRows, rows, a.sliceMax, dc, cg, smem);
-                    ++g_kernelLaunches;
-                    CIPC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(nbRows), dim3(threads), args, smem, c.s));
-                    return;
+            for (int rows = std::max(SINGLE_MIN_ROWS, even), last = 0; !last; rows = std::max(even, rows / 2)) {
+                last = !LEARNED || rows == even;
+                const int threads = std::min(PB, std::max(256, (rows * GROUP + 31) / 32 * 32));  // half a block at least, to stage wide rows
+                const int nbRows = (c.nv + rows - 1) / rows;
+                a.rowsPerBlock = rows;
+                a.sliceMax = pcgSliceMax(c, rows);
+                for (int dc : dynCaps) {
+                    if (!dyn && dc > 0) continue;
+                    size_t smem = smemLayout(a.sliceMax, dc, cg != 0, (int)sizeof(MT), (int)sizeof(VT)).total;
+                    if (smem + 4096 > (size_t)maxOptin) continue;
+                    int perSM = 0;
+                    CIPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, threads, smem));
+                    if (perSM >= 1 && nbRows <= perSM * smCount && nbRows <= cap) {
+                        a.dynCap = dc;
+                        a.cacheG = cg;
+                        if (debugPcg())
+                            std::fprintf(stderr, "[pcg] single-pass launch: %d blocks of %d rows, slice %d, contact window %d, factor cached %d, %zu B shared\n",
+                                         nbRows, rows, a.sliceMax, dc, cg, smem);
+                        ++g_kernelLaunches;
+                        CIPC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(nbRows), dim3(threads), args, smem, c.s));
+                        return;
+                    }
                 }
             }
         }

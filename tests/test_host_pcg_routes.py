@@ -1,0 +1,51 @@
+"""Which PCG kernel a system goes to."""
+import numpy as np
+import pytest
+
+import fake_runtime
+
+KERNELS = ("pcgPipelinedKernel", "pcgStreamKernel", "pcgPersistentKernel")
+
+
+@pytest.fixture(scope="module")
+def fake():
+    return fake_runtime.runtime()
+
+
+def launched(fake):
+    """The last solve's kernel, with its mangled arguments, and its grid."""
+    launch = [e for e in fake.events("launch") if any(k in e for k in KERNELS)][-1]
+    return launch.split()[1], int(launch.split(" grid ")[1].split()[0])
+
+
+def tangle(fake, nv, tets, seed=3):
+    """A context of tetrahedra between any of nv points: every row is wide."""
+    rng = np.random.default_rng(seed)
+    scene = fake.cipc.scene_two_cubes(1)
+    x = rng.random((nv, 3))
+    t = np.array([rng.choice(nv, 4, replace=False) for _ in range(tets)], np.int32)
+    e = x[t[:, 1:]] - x[t[:, :1]]
+    flip = np.linalg.det(e) < 0
+    t[flip, 2:] = t[flip, 2:][:, ::-1]
+    scene.update(x=x, tets=t, btype=np.zeros(nv, np.int32))
+    return fake.cipc.Simulator(scene, precond="fsai")
+
+
+@pytest.mark.parametrize("nv,tets,rows", [(443, 500, 64), (443, 2000, 16), (443, 8000, 8)])
+def test_factor_of_wide_rows_stays_in_one_pass(fake, nv, tets, rows):
+    """Where 64 rows and their factor do not fit a block, fewer do: the factor is
+    then read in FP32, which the streaming kernel's tiles would round to FP16."""
+    sim = tangle(fake, nv, tets)
+    sim.assemble()
+    fake.reset()
+    sim.solve()
+    name, grid = launched(fake)
+    sim.close()
+    assert "pcgPipelinedKernelIddLb1E" in name
+    assert grid == -(-nv // rows)
+
+
+def test_rows_that_fit_no_block_stream(fake):
+    fake.reset()
+    fake.cipc.pcg_bsr(*fake_runtime.ring_system(9001, range(1, 31)))
+    assert "pcgStreamKernel" in launched(fake)[0]
