@@ -710,11 +710,16 @@ __global__ void __launch_bounds__(PB) pcgPersistentKernel(PcgArgs<MT, VT> a) {
 // gathered vectors from L2.
 constexpr int ROWS_PER_BLOCK = PB / GROUP;
 // Rows per block of a small system: fewer and fuller blocks make the grid
-// barrier and its sums cheaper.  Measured per solve on a B200 with at least 3 (one
-// block per SM), 16, 32 and 64 rows: 432 rows 2.78, 2.63, 2.62, 2.58 ms; 1,881
-// rows (13 a block) 0.29, 0.30, 0.27, 0.26 ms; 1,458 FP32 rows 4.55, 4.33, 4.38,
-// 4.19 ms.
-constexpr int SINGLE_MIN_ROWS = 64;
+// barrier and its sums cheaper, until the SMs left idle cost more.  Up to
+// SINGLE_FILL_ROWS rows a block in an even spread over the SMs a block takes
+// SINGLE_MIN_ROWS, beyond that the even share.  Measured per solve on a B200, with 64
+// rows a block and with the even share (in brackets), ms:
+//   even share 3-30: 432 rows 2.59 (2.77), 1,458 FP32 4.22 (4.61), 1,881 0.25
+//   (0.27), 2,000 3.82 (4.22), 2,662 with a factor 6.35 (6.46), 4,329 0.49 (0.51),
+//   4,394 4.09 (4.14);
+//   even share 41-54: 6,001 0.49 (0.49), 6,750 4.55 (4.20), 6,932 2.38 (2.40),
+//   7,954 FP32 1.05 (1.00), 8,001 0.56 (0.52).
+constexpr int SINGLE_MIN_ROWS = 64, SINGLE_FILL_ROWS = 32;
 constexpr int STATE_VECS = 9;  // x r u w z q s p, and the row's own m
 
 struct SmemLayout {
@@ -1812,8 +1817,8 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
         // stages them in shared memory.  The largest configuration that keeps
         // every block resident is taken: the factor's blocks cached or not, a
         // contact window of 512 down to 0 slots.  Rows are spread evenly over one
-        // block per SM or more, SINGLE_MIN_ROWS at least.  Where so many wide rows
-        // do not fit, the streaming kernel takes a block-Jacobi solve as fast (443
+        // block per SM or more, in a small system SINGLE_MIN_ROWS.  Where so many wide
+        // rows do not fit, the streaming kernel takes a block-Jacobi solve as fast (443
         // rows of 161 blocks on a B200: 0.59 ms with 8 rows a block, 0.58 streamed;
         // FP32 0.74 and 0.51); a factor, which it would round to FP16, stays here
         // with fewer rows a block, down to the even spread.
@@ -1826,7 +1831,7 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
         const bool dyn = a.dRowS != nullptr;
         static const int dynCaps[] = {512, 256, 128, 0};
         for (int cg = LEARNED ? 1 : 0; cg >= 0; --cg) {
-            for (int rows = std::max(SINGLE_MIN_ROWS, even), last = 0; !last; rows = std::max(even, rows / 2)) {
+            for (int rows = even <= SINGLE_FILL_ROWS ? SINGLE_MIN_ROWS : even, last = 0; !last; rows = std::max(even, rows / 2)) {
                 last = !LEARNED || rows == even;
                 const int threads = std::min(PB, std::max(256, (rows * GROUP + 31) / 32 * 32));  // half a block at least, to stage wide rows
                 const int nbRows = (c.nv + rows - 1) / rows;

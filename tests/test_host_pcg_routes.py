@@ -49,3 +49,13 @@ def test_rows_that_fit_no_block_stream(fake):
     fake.reset()
     fake.cipc.pcg_bsr(*fake_runtime.ring_system(9001, range(1, 31)))
     assert "pcgStreamKernel" in launched(fake)[0]
+
+
+@pytest.mark.parametrize("nv,rows", [(1, 64), (443, 64), (4736, 64), (4737, 33), (9001, 61), (9473, 65), (18944, 128)])
+def test_rows_per_block(fake, nv, rows):
+    """64 rows a block while an even spread over the 148 SMs has at most 32."""
+    fake.reset()
+    fake.cipc.pcg_bsr(*fake_runtime.ring_system(nv))
+    name, grid = launched(fake)
+    assert "pcgPipelinedKernel" in name
+    assert grid == -(-nv // rows)
