@@ -140,7 +140,7 @@ struct DevBvh {
 struct SellRows {
     DBuf<int> ptr, slot, tile, col;
     DBuf<unsigned char> val;
-    int steps = 0;
+    int steps = 0, longest = 0;          // in all, and of the longest tile
     bool laid = false, hasCols = false;  // offsets and columns are in place
     void free() { ptr.free(); slot.free(); tile.free(); col.free(); val.free(); }
 };

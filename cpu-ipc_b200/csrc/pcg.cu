@@ -1141,6 +1141,18 @@ constexpr int streamWarps(bool beyond) { return beyond ? 24 : 16; }
 // Beyond when an iteration's data exceed this share of L2 (63 MB): 27-cube pile,
 // 45 MB, 7.9 ms within and 9.2 beyond; with the factor, 75 MB, 11.8 and 10.9.
 constexpr double STREAM_L2_SHARE = 0.5;
+// Tiles suit rows that are alike: their steps past each tile's first (which is
+// there even for a single block) hold at most SELL_PAD slots per block.  The meshes of
+// the scenes are at 0.8-1.15.  Past it tiles still suit if they lie within L2 and no
+// tile is longer than SELL_LONG steps.  Measured per iteration on a B200 in tiles and in
+// block-CSR rows (pcgRowsKernel), us, FP64 and FP32 blocks, 40,011 rows unless said:
+//   every 8th row joined to 24 others 12.7 and 17.1, 11.8 and 14.9; every 2nd to 30
+//   17.0 and 24.4, 15.5 and 20.3 (within L2: 53-118 MB); every 8th to 60 32 and
+//   25 (203 MB), 20.9 and 21.0 (111 MB); every 32nd to 100 (26 steps) 21.8 and 20.4,
+//   24.4 and 20.2; every 2nd to 200 151 and 96, 96 and 79; 200,011 rows, every 8th to 12
+//   66 and 53, 52 and 42 (170 MB).
+constexpr double SELL_PAD = 1.5;
+constexpr int SELL_LONG = 16;
 constexpr size_t STREAM_STATE_BYTES = 192 * 1024;  // recurrence vectors in shared memory, per SM
 
 // fetch [p, p + bytes) into L2 (both multiples of 16)
@@ -1567,6 +1579,124 @@ __global__ void __launch_bounds__(32 * streamWarps(BEYOND), 1) pcgStreamKernel(P
     }
 }
 
+// The same recurrences with block-Jacobi over block-CSR rows in memory, for
+// patterns whose rows differ so much that tiles would be mostly padding
+// (SELL_PAD).  A row of some hundred blocks is a chain of loads, so this build
+// keeps three blocks of 512 threads on an SM (40 registers) and deals the rows of
+// the whole system out in turn.  Measured per iteration on a B200, FP64, here and in
+// tiles: 40,011 rows, every 8th joined to 200 others, 50 and 100 us, every 32nd to
+// 400, 44 and 141; 200,011 rows, every 8th joined to 80, 101 and 238.  Bound by the
+// longest row's chain and by nine scattered loads a block.
+template <class MT>
+__global__ void __launch_bounds__(PB, 3) pcgRowsKernel(PcgArgs<MT, double> a) {
+    const unsigned nb = gridDim.x;
+    unsigned ep = 0;
+    const int nv = a.nv;
+    const RowIter it;
+    const int q = it.lane;  // the component this lane updates (q < 3)
+    auto part = [&](int set, int k) { return a.pp + (size_t)(3 * set + k) * PIPE_PMAX; };
+    auto pick = [&](const double v[3]) { return q == 0 ? v[0] : (q == 1 ? v[1] : v[2]); };
+    auto rowDot = [&](const double* D, const double v[3]) { return D[3 * q] * v[0] + D[3 * q + 1] * v[1] + D[3 * q + 2] * v[2]; };
+    // m = Dinv v for the row, v held by lanes 0, 1, 2 of its group; every lane calls
+    auto precondRow = [&](int row, double vq, double* out) {
+        const double v[3] = {__shfl_sync(0xffffffffu, vq, 0, GROUP), __shfl_sync(0xffffffffu, vq, 1, GROUP), __shfl_sync(0xffffffffu, vq, 2, GROUP)};
+        double o = 0.0;
+        if (row < nv && q < 3) out[3 * (size_t)row + q] = o = rowDot(a.Dinv + 9 * (size_t)row, v);
+        return o;
+    };
+    // x = 0, r = b, u = M r; the recurrence vectors start at 0
+    double rr = 0, g = 0, dl = 0;
+    for (int base = it.first; base < nv; base += it.stride) {
+        const int row = base + it.grp;
+        const size_t i = 3 * (size_t)row + q;
+        double rq = 0.0;
+        if (row < nv && q < 3) {
+            a.x[i] = a.z[i] = a.q[i] = a.s[i] = a.p[i] = 0.0;
+            a.r[i] = rq = a.b[i];
+            rr += rq * rq;
+        }
+        precondRow(row, rq, a.u);
+    }
+    if (!gridBarrier(a.bar, a.flag, nb, ep)) return;
+    // w = A u, m = M w, gamma = (r,u), delta = (w,u).  The recurrences overwrite
+    // u row by row while its neighbours still read m alone.
+    for (int base = it.first; base < nv; base += it.stride) {
+        const int row = base + it.grp;
+        const size_t i = 3 * (size_t)row + q;
+        double acc[3] = {0.0, 0.0, 0.0};
+        if (row < nv) rowSpmv(a, row, q, (const double*)a.u, acc);
+        groupReduce3(acc);
+        double wq = 0.0;
+        if (row < nv && q < 3) {
+            const double uo[3] = {a.u[3 * (size_t)row], a.u[3 * (size_t)row + 1], a.u[3 * (size_t)row + 2]};
+            a.w[i] = wq = pick(acc) + rowDot(a.diagExtra + 9 * (size_t)row, uo);
+            g += a.r[i] * pick(uo);
+            dl += wq * pick(uo);
+        }
+        precondRow(row, wq, a.mA);
+    }
+    blockReduce3(rr, g, dl);
+    if (threadIdx.x == 0) { part(0, 0)[blockIdx.x] = rr; part(0, 1)[blockIdx.x] = g; part(0, 2)[blockIdx.x] = dl; }
+    double sums[3];  // r.r, gamma, delta
+    if (!gridBarrierSum<3>(a.bar, a.flag, nb, ep, part(0, 0), PIPE_PMAX, sums)) return;
+    const double rhs2 = sums[0];
+    const double thr = fmax(a.tol * a.tol * rhs2, 2.2250738585072014e-308);
+    int iter = 0;
+    int status = (rhs2 == 0.0 || rhs2 < thr) ? 1 : 0;
+    double gPrev = 1.0, alPrev = 1.0;
+    while (status == 0) {
+        g = sums[1];
+        const double bt = iter == 0 ? 0.0 : g / gPrev;
+        const double den = iter == 0 ? sums[2] : sums[2] - bt * g / alPrev;
+        if (!(den != 0.0) || !isfinite(den)) { status = 2; break; }  // breakdown: the caller's true residual decides
+        const double al = g / den;
+        const double* mCur = (iter & 1) == 0 ? a.mA : a.mB;
+        double* mNext = (iter & 1) == 0 ? a.mB : a.mA;
+        double lrr = 0, lg = 0, ld = 0;
+        for (int base = it.first; base < nv; base += it.stride) {
+            const int row = base + it.grp;
+            const size_t i = 3 * (size_t)row + q;
+            double acc[3] = {0.0, 0.0, 0.0};
+            if (row < nv) rowSpmv(a, row, q, mCur, acc);
+            groupReduce3(acc);
+            double wq = 0.0;
+            if (row < nv && q < 3) {
+                const double mo[3] = {mCur[3 * (size_t)row], mCur[3 * (size_t)row + 1], mCur[3 * (size_t)row + 2]};
+                const double zv = pick(acc) + rowDot(a.diagExtra + 9 * (size_t)row, mo) + bt * a.z[i];
+                const double qv = pick(mo) + bt * a.q[i];
+                const double w0 = a.w[i], u0 = a.u[i];
+                const double sq = w0 + bt * a.s[i];
+                const double pv = u0 + bt * a.p[i];
+                a.z[i] = zv; a.q[i] = qv; a.s[i] = sq; a.p[i] = pv;
+                a.x[i] += al * pv;
+                const double rv = a.r[i] - al * sq;
+                const double uv = u0 - al * qv;
+                wq = w0 - al * zv;
+                a.r[i] = rv; a.u[i] = uv; a.w[i] = wq;
+                lrr += rv * rv;
+                lg += rv * uv;
+                ld += wq * uv;
+            }
+            precondRow(row, wq, mNext);
+        }
+        const int set = (iter + 1) & 1;
+        blockReduce3(lrr, lg, ld);
+        if (threadIdx.x == 0) { part(set, 0)[blockIdx.x] = lrr; part(set, 1)[blockIdx.x] = lg; part(set, 2)[blockIdx.x] = ld; }
+        if (!gridBarrierSum<3>(a.bar, a.flag, nb, ep, part(set, 0), PIPE_PMAX, sums)) return;
+        gPrev = g;
+        alPrev = al;
+        ++iter;
+        if (sums[0] < thr) { status = 1; break; }
+        if (iter >= a.maxIter || !isfinite(sums[0])) { status = 2; break; }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.scal[3] = sums[0];
+        a.scal[4] = iter;
+        a.scal[6] = rhs2;
+        atomicCAS(a.flag, 0, status);  // a barrier timeout (3) stands
+    }
+}
+
 __global__ void accumulateKernelD(int n3, const double* d, double* x) {
     CIPC_KERNEL_LOOP(i, n3) x[i] += d[i];
 }
@@ -1609,17 +1739,41 @@ __global__ void packTilesKernel(int nv, const int* ptr, const int* slotOf, const
     }
 }
 
-// Step offsets of the tiles of 8 rows with the given row offsets.
+// Steps of tile t of 8 rows with the given row offsets.
+static int tileSteps(int nv, const std::vector<int>& ptr, int t) {
+    int most = 0;
+    for (int r = 8 * t; r < std::min(nv, 8 * t + 8); ++r) most = std::max(most, ptr[r + 1] - ptr[r]);
+    return (most + GROUP - 1) / GROUP;
+}
+
+// Step offsets of the tiles.
 static void tileOffsets(Ctx& c, SellRows& m, int nv, const std::vector<int>& ptr) {
     std::vector<int> tile((nv + 7) / 8 + 1, 0);
-    for (int t = 0; 8 * t < nv; ++t) {
-        int steps = 0;
-        for (int r = 8 * t; r < std::min(nv, 8 * t + 8); ++r) steps = std::max(steps, (ptr[r + 1] - ptr[r] + GROUP - 1) / GROUP);
-        tile[t + 1] = tile[t] + steps;
-    }
+    for (int t = 0; 8 * t < nv; ++t) tile[t + 1] = tile[t] + tileSteps(nv, ptr, t);
     m.steps = tile.back();
     upload(c, m.tile, tile);
     m.laid = true;
+}
+
+// What a block-Jacobi iteration over the tiles reads: matrix, gathered vectors
+// and diagonal blocks.
+static double tileBytes(const Ctx& c, size_t valueSize) { return (double)c.sellA.steps * (288 * valueSize + 128) + c.nv * (2 * 72.0 + 2 * 32.0); }
+
+// Whether the static pattern goes into tiles (SELL_PAD).
+static bool rowsSuitTiles(Ctx& c) {
+    SellRows& m = c.sellA;
+    const int tiles = (c.nv + 7) / 8;
+    if (!m.steps)
+        for (int t = 0; t < tiles; ++t) {
+            const int n = tileSteps(c.nv, c.hRowPtr, t);
+            m.steps += n;
+            m.longest = std::max(m.longest, n);
+        }
+    if (32.0 * (m.steps - tiles) <= SELL_PAD * c.nnzb) return true;
+    int dev = 0, l2 = 0;
+    CIPC_CUDA(cudaGetDevice(&dev));
+    CIPC_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+    return m.longest <= SELL_LONG && tileBytes(c, c.mixed ? sizeof(float) : sizeof(double)) <= l2;
 }
 
 template <class MT, class OT>
@@ -1869,6 +2023,20 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
         CIPC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(PB), args, 0, c.s));
         return;
     }
+    if constexpr (sizeof(VT) == sizeof(double) && !LEARNED) {
+        // (a factor belongs to a mesh, whose rows are alike)
+        if (!rowsSuitTiles(c)) {
+            const void* fn = (const void*)pcgRowsKernel<MT>;
+            int perSM = 0;
+            CIPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, PB, 0));
+            if (perSM < 1) throw std::runtime_error("streaming PCG kernel does not fit on an SM");
+            const int grid = std::max(1, std::min(std::min(std::min(perSM, 3) * smCount, needed), cap));
+            if (debugPcg()) std::fprintf(stderr, "[pcg] block-CSR launch: %d blocks, %d tile steps for %d blocks\n", grid, c.sellA.steps, c.nnzb);
+            ++g_kernelLaunches;
+            CIPC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(PB), args, 0, c.s));
+            return;
+        }
+    }
     if constexpr (sizeof(VT) == sizeof(double)) {
         const bool half = LEARNED && !pcgNoPack();
         if (half) packStream<MT, __half>(c, a.val, true);
@@ -1890,7 +2058,7 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
         a.state = c.pcgState.p;
         // what every iteration reads: matrix, factor, gathered vectors, diagonal
         // blocks and the state
-        double bytes = (double)c.sellA.steps * (288 * sizeof(MT) + 128) + c.nv * (2 * 72.0 + 2 * 32.0) + (a.resident ? 0.0 : (double)state * grid);
+        double bytes = tileBytes(c, sizeof(MT)) + (a.resident ? 0.0 : (double)state * grid);
         if (LEARNED) bytes += ((double)c.sellL.steps + c.sellU.steps) * (288.0 * (half ? 2 : 4) + 128) + c.nv * 32.0;
         int dev = 0, l2 = 0;
         CIPC_CUDA(cudaGetDevice(&dev));
@@ -2175,15 +2343,9 @@ void lendPcg(Ctx& c, DevSlab& slab) {
     int dev = 0, sms = 0;
     CIPC_CUDA(cudaGetDevice(&dev));
     CIPC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (nv > (size_t)sms * ROWS_PER_BLOCK) {
+    if (nv > (size_t)sms * ROWS_PER_BLOCK && rowsSuitTiles(c)) {
         // more rows than the single-pass launch can hold: the tiles too
         const size_t tiles = (nv + 7) / 8;
-        if (!c.sellA.steps)
-            for (size_t t = 0; t < tiles; ++t) {
-                int most = 0;
-                for (size_t r = 8 * t; r < std::min(nv, 8 * t + 8); ++r) most = std::max(most, c.hRowPtr[r + 1] - c.hRowPtr[r]);
-                c.sellA.steps += (most + GROUP - 1) / GROUP;
-            }
         slab.lend(c.sellA.tile, tiles + 1);
         slab.lend(c.sellA.col, 32 * (size_t)c.sellA.steps);
         slab.lend(c.sellA.val, 288 * (c.mixed ? sizeof(float) : sizeof(double)) * (size_t)c.sellA.steps);

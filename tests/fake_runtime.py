@@ -59,6 +59,19 @@ def ring_system(nv, neighbours=(1, 2, 5)):
     distances (the values do not matter: kernels do not run)."""
     i = np.arange(nv)
     pairs = np.concatenate([np.stack([i, (i + d) % nv]) for d in (0,) + tuple(neighbours) + tuple(-d for d in neighbours)], axis=1)
+    return _blocks(nv, pairs)
+
+
+def hub_system(nv, every, degree):
+    """As ring_system, a ring with every `every`-th row joined to `degree` others of them."""
+    i = np.arange(nv)
+    h = i[::every]
+    to = [np.stack([i, (i + d) % nv]) for d in (0, 1, -1)]
+    to += [np.stack([h, np.roll(h, d)]) for k in range(1, degree // 2 + 1) for d in (k, -k)]
+    return _blocks(nv, np.concatenate(to, axis=1))
+
+
+def _blocks(nv, pairs):
     key = np.unique(pairs[0].astype(np.int64) * nv + pairs[1])
     rp = np.concatenate([[0], np.cumsum(np.bincount(key // nv, minlength=nv))]).astype(np.int32)
     return rp, (key % nv).astype(np.int32), np.zeros((len(key), 3, 3)), np.zeros(3 * nv)

@@ -4,7 +4,7 @@ import pytest
 
 import fake_runtime
 
-KERNELS = ("pcgPipelinedKernel", "pcgStreamKernel", "pcgPersistentKernel")
+KERNELS = ("pcgPipelinedKernel", "pcgStreamKernel", "pcgPersistentKernel", "pcgRowsKernel")
 
 
 @pytest.fixture(scope="module")
@@ -59,3 +59,17 @@ def test_rows_per_block(fake, nv, rows):
     name, grid = launched(fake)
     assert "pcgPipelinedKernel" in name
     assert grid == -(-nv // rows)
+
+
+@pytest.mark.parametrize("every,degree,tiles", [
+    (8, 0, True), (8, 12, True), (8, 24, True), (2, 30, True), (1, 200, True), (400, 200, True),
+    (8, 60, False), (2, 200, False), (8, 200, False), (16, 100, False), (32, 100, False)])
+def test_padding_of_tiles(fake, every, degree, tiles):
+    """Where the rows of a tile differ so much that most of its slots would be
+    empty, and they are many or in long chains, the block-CSR rows are read as
+    they are, and no tiles are stored."""
+    system = fake_runtime.hub_system(40011, every, degree)
+    fake.reset()
+    fake.cipc.pcg_bsr(*system)
+    assert ("pcgStreamKernel" if tiles else "pcgRowsKernel") in launched(fake)[0]
+    assert len(fake.events("launch", "packTilesKernel")) == int(tiles)
