@@ -61,8 +61,9 @@ struct DBuf {
     bool lent = false;  // p is a piece of a DevSlab
     // grows to twice the request: buffers sized by contact counts grow for a
     // few steps and then stay (a reallocation costs a device-wide wait and
-    // page mapping, tens of milliseconds for the pile's contact buffers)
-    void reserve(size_t n) {
+    // page mapping, tens of milliseconds for the pile's contact buffers).  exact:
+    // to the request itself, for buffers whose size the mesh fixes
+    void reserve(size_t n, bool exact = false) {
         if (n <= cap) return;
         const bool dbg = debugAlloc();
         const auto t0 = dbg ? std::chrono::steady_clock::now() : std::chrono::steady_clock::time_point();
@@ -71,7 +72,7 @@ struct DBuf {
         p = nullptr;
         const size_t old = cap;
         cap = 0;  // until the allocation has succeeded
-        size_t c = n < 64 ? 64 : 2 * n;
+        size_t c = exact ? n : n < 64 ? 64 : 2 * n;
         CIPC_CUDA(cudaMalloc(&p, c * sizeof(T)));
         if (dbg) reportAlloc(old * sizeof(T), c * sizeof(T), std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
         cap = c;

@@ -297,13 +297,13 @@ struct PcgArgs {
     VT* t;
     const VT* b;
     VT *x, *r, *z, *p, *Ap;
-    VT *u, *w, *mA, *mB, *q, *s;  // pipelined variants only
+    VT *u, *w, *mA, *mB, *q, *s;  // pipelined variants over block-CSR rows only
     // streaming variant: gathered vectors padded to 4 entries per row, the
-    // tiled matrix and factor parts, the tiles a block owns at most, whether
-    // the recurrence vectors live in shared memory, and else where they live
+    // tiled matrix and factor parts, whether the recurrence vectors live in
+    // shared memory, and else where they live
     VT *g0, *g1, *g2, *g3, *state;
     SellView sA, sL, sU;
-    int resident, tilesPerBlock;
+    int resident;
     double *partA, *partB, *partC;
     double* pp;                   // pipelined variant: two sets of three partial arrays, PIPE_PMAX each
     int sliceMax;                 // cached variant: static slots of the largest block row range
@@ -1779,8 +1779,8 @@ static bool rowsSuitTiles(Ctx& c) {
 template <class MT, class OT>
 static void packTiles(Ctx& c, SellRows& m, const int* ptr, const int* slotOf, const MT* src) {
     const bool first = !m.hasCols;
-    m.col.reserve(std::max<size_t>((size_t)32 * m.steps, 1));
-    m.val.reserve(std::max<size_t>((size_t)288 * sizeof(OT) * m.steps, 16));
+    m.col.reserve(std::max<size_t>((size_t)32 * m.steps, 1), true);
+    m.val.reserve(std::max<size_t>((size_t)288 * sizeof(OT) * m.steps, 16), true);
     const int nb = std::max(1, std::min(((c.nv + 7) / 8 + VB / 32 - 1) / (VB / 32), 148 * 8));
     launch(packTilesKernel<MT, OT>, nb, VB, 0, c.s, c.nv, ptr, slotOf, (const int*)c.colIdx, src, (const int*)m.tile, first ? m.col.p : (int*)nullptr,
            reinterpret_cast<OT*>(m.val.p));
@@ -1959,6 +1959,16 @@ static void allowSharedMemory(const void* fn) {
     CIPC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
 }
 
+// The six vectors that the pipelined kernels over block-CSR rows keep beside the
+// caller's.
+template <class MT, class VT>
+static void pipeVectors(Ctx& c, PcgArgs<MT, VT>& a) {
+    const size_t n3 = 3 * (size_t)c.nv;
+    c.pcgPipe.reserve(6 * n3 * sizeof(VT) / sizeof(double) + 6);
+    VT* pv = reinterpret_cast<VT*>(c.pcgPipe.p);
+    a.u = pv; a.w = pv + n3; a.mA = pv + 2 * n3; a.mB = pv + 3 * n3; a.q = pv + 4 * n3; a.s = pv + 5 * n3;
+}
+
 template <class MT, class VT, bool LEARNED>
 static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool classic) {
     int needed = std::max(1, (c.nv * GROUP + PB - 1) / PB);
@@ -2000,6 +2010,7 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
                     if (perSM >= 1 && nbRows <= perSM * smCount && nbRows <= cap) {
                         a.dynCap = dc;
                         a.cacheG = cg;
+                        pipeVectors(c, a);
                         if (debugPcg())
                             std::fprintf(stderr, "[pcg] single-pass launch: %d blocks of %d rows, slice %d, contact window %d, factor cached %d, %zu B shared\n",
                                          nbRows, rows, a.sliceMax, dc, cg, smem);
@@ -2031,6 +2042,7 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
             CIPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, PB, 0));
             if (perSM < 1) throw std::runtime_error("streaming PCG kernel does not fit on an SM");
             const int grid = std::max(1, std::min(std::min(std::min(perSM, 3) * smCount, needed), cap));
+            pipeVectors(c, a);
             if (debugPcg()) std::fprintf(stderr, "[pcg] block-CSR launch: %d blocks, %d tile steps for %d blocks\n", grid, c.sellA.steps, c.nnzb);
             ++g_kernelLaunches;
             CIPC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(PB), args, 0, c.s));
@@ -2045,16 +2057,16 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
         a.sA = view(c.sellA); a.sL = view(c.sellL); a.sU = view(c.sellU);
         // padded gathered vectors
         const size_t n4 = 4 * (size_t)c.nv;
-        c.pcgGather.reserve(4 * n4);
+        c.pcgGather.reserve(4 * n4, true);
         a.g0 = c.pcgGather.p; a.g1 = a.g0 + n4; a.g2 = a.g1 + n4; a.g3 = a.g2 + n4;
         const int tiles = (c.nv + 7) / 8;
         const int grid = std::max(1, std::min(std::min(smCount, tiles), cap));
-        a.tilesPerBlock = (tiles + grid - 1) / grid;
+        const int tilesPerBlock = (tiles + grid - 1) / grid;  // at most
         // the state vectors in shared memory where all eight fit
-        const size_t state = (size_t)a.tilesPerBlock * 24 * sizeof(double) * 8;
+        const size_t state = (size_t)tilesPerBlock * 24 * sizeof(double) * 8;
         a.resident = state <= STREAM_STATE_BYTES ? 1 : 0;
         const size_t smem = a.resident ? state : 0;
-        if (!a.resident) c.pcgState.reserve(8 * (size_t)tiles * 24);
+        if (!a.resident) c.pcgState.reserve(8 * (size_t)tiles * 24, true);
         a.state = c.pcgState.p;
         // what every iteration reads: matrix, factor, gathered vectors, diagonal
         // blocks and the state
@@ -2071,7 +2083,7 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
         int fit = 0;
         CIPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, threads, smem));
         if (fit * smCount < grid) throw std::runtime_error("streaming PCG kernel does not fit on an SM");
-        if (debugPcg()) std::fprintf(stderr, "[pcg] streaming launch: %d blocks of %d tiles, state in shared memory %d, beyond L2 %d (%.1f MB)\n", grid, a.tilesPerBlock, a.resident, (int)beyond, bytes * 1e-6);
+        if (debugPcg()) std::fprintf(stderr, "[pcg] streaming launch: %d blocks of %d tiles, state in shared memory %d, beyond L2 %d (%.1f MB)\n", grid, tilesPerBlock, a.resident, (int)beyond, bytes * 1e-6);
         ++g_kernelLaunches;
         CIPC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem, c.s));
     }
@@ -2104,11 +2116,7 @@ static int runPcgPersistent(Ctx& c, const MT* val, const MT* dval, const VT* b, 
         a.S = c.mpS.p; a.gS = c.mpGS.p; a.gD = c.mpGD.p; a.t = reinterpret_cast<VT*>(c.mpT.p);
     }
     a.partA = c.red.p; a.partB = c.red.p + PMAX; a.partC = c.red.p + 2 * PMAX;
-    // pipelined kernel: six more vectors and two sets of partial sums
-    size_t n3 = 3 * (size_t)c.nv;
-    c.pcgPipe.reserve(6 * n3 * sizeof(VT) / sizeof(double) + 6);
-    VT* pv = reinterpret_cast<VT*>(c.pcgPipe.p);
-    a.u = pv; a.w = pv + n3; a.mA = pv + 2 * n3; a.mB = pv + 3 * n3; a.q = pv + 4 * n3; a.s = pv + 5 * n3;
+    // pipelined kernels: two sets of partial sums
     c.pcgParts.reserve(6 * (size_t)PIPE_PMAX);
     a.pp = c.pcgParts.p;
     a.scal = c.scal.p; a.flag = c.counters.p + 10;
@@ -2337,14 +2345,16 @@ void lendPcg(Ctx& c, DevSlab& slab) {
     slab.lend(c.rF, n3);
     if (c.mixed)
         for (DBuf<float>* d : {&c.zF, &c.pF, &c.ApF, &c.xF, &c.DinvF}) slab.lend(*d, n3);
-    slab.lend(c.pcgPipe, 6 * n3 + 6);
     slab.lend(c.pcgParts, 6 * (size_t)PIPE_PMAX);
     slab.lend(c.pcgBar, BAR_WORDS);
     int dev = 0, sms = 0;
     CIPC_CUDA(cudaGetDevice(&dev));
     CIPC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (nv > (size_t)sms * ROWS_PER_BLOCK && rowsSuitTiles(c)) {
-        // more rows than the single-pass launch can hold: the tiles too
+    const bool single = nv <= (size_t)sms * ROWS_PER_BLOCK, rows = !single && !rowsSuitTiles(c);
+    if (single || rows) {
+        slab.lend(c.pcgPipe, 6 * n3 + 6);
+    } else {
+        // more rows than a single-pass launch of one block per SM can hold
         const size_t tiles = (nv + 7) / 8;
         slab.lend(c.sellA.tile, tiles + 1);
         slab.lend(c.sellA.col, 32 * (size_t)c.sellA.steps);

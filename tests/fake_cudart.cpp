@@ -5,7 +5,7 @@
 //   - a host-to-device copy or fill on the legacy stream counts as under way
 //     until that stream is waited for, and a kernel launched on another stream
 //     meanwhile is noted as unordered;
-//   - cudaMalloc can be made to fail;
+//   - cudaMalloc's sizes are noted, and it can be made to fail;
 //   - a launch asking for more dynamic shared memory than the kernel's
 //     attribute allows is refused.
 #include <cuda_runtime_api.h>
@@ -88,6 +88,7 @@ cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3 g, dim3 b, void** a,
 cudaError_t cudaMalloc(void** p, size_t n) {
     std::lock_guard<std::recursive_mutex> lock(mu);
     ++mallocs;
+    note("malloc " + std::to_string(n));
     if (failIn && --failIn == 0) return fail(cudaErrorMemoryAllocation);
     *p = std::calloc(std::max<size_t>(n, 1), 1);
     live[*p] = n;

@@ -32,4 +32,5 @@ def test_tiles_of_a_solve_that_failed_are_laid_out_again(precond):
         sim.solve()
         assert len(fake.events("launch", "columns 1")) == sets, nth
         sim.close()
+    fake.L.fake_fail_malloc(0)
     assert failures > 10
