@@ -368,7 +368,6 @@ void finalizeDynamic(Ctx& c);          // sort + segment dynamic gradient and He
 
 // ---- launchers (pcg.cu) ----
 int pcgSolve(Ctx& c);                  // solves A sol = rhs; returns iterations
-void spmv(Ctx& c, const double* x, double* y);
 void buildRhs(Ctx& c);
 void lendPcg(Ctx& c, DevSlab& slab);   // every buffer of a block-Jacobi solve
 void roundBlocks(Ctx& c, size_t n, const double* src, float* dst);

@@ -4,16 +4,13 @@
 // backends (CPU IPC/NewtonLinearSystem.cpp:21-56, 176-207).  The stopping rule
 // is Eigen's: ||r||^2 < tol^2 ||b||^2 with x0 = 0.
 //
-// SpMV: a group of 8 lanes owns one block row; lanes stride over the row's
-// 3x3 blocks (contiguous 72-byte FP64 or 36-byte FP32 blocks, so a group reads
-// one coalesced run) and combine with shuffles.  Dot products reduce per block
-// into partials; the next kernel sums the partials in a fixed order, so no
-// host round trip is needed inside an iteration and results are reproducible.
+// A solve is one cooperative launch: rows staged in shared memory where they fit,
+// else streamed in tiles or as block-CSR rows.  Groups of 4 lanes own block rows
+// and combine with shuffles; partial sums are added in a fixed order, so no host
+// round trip is needed inside an iteration and results are reproducible.
 //
-// Mixed precision: FP32 blocks, FP32 vectors and FP32 SpMV accumulation in an
-// inner PCG, wrapped in FP64 iterative refinement: the outer loop recomputes
-// the true residual b - A x in FP64 (FP32 blocks promoted) and stops on the
-// same FP64 criterion as the FP64 solver.
+// Mixed precision: FP32 blocks, FP64 vectors; the stopping rule is decided on the
+// true residual b - A x in FP64 (FP32 blocks promoted).
 #include "cipc_device.cuh"
 #include <cuda_fp16.h>
 #include "cipc_gpu.h"
@@ -59,14 +56,12 @@ __device__ __forceinline__ void blockMulAddH(const __half* B, const VT* xv, VT a
 // y = A x ; partial[block] = sum over the block's rows of x . y (for p.Ap)
 template <class MT, class VT>
 __global__ void spmvKernel(int nv, const int* rowPtr, const int* col, const MT* val, const int* dRowS, const int* dRowE, const int* dCol,
-                           const MT* dVal, const double* diagExtra, const VT* x, VT* y, double* partial, const int* flag) {
-    if (flag && *flag) return;
+                           const MT* dVal, const double* diagExtra, const VT* x, VT* y) {
     int gid = blockIdx.x * blockDim.x + threadIdx.x;
     int lane = threadIdx.x & (GROUP - 1);
     int grp = (threadIdx.x & 31) / GROUP;
     const int RPW = 32 / GROUP;  // rows per warp per pass
     int nWarps = gridDim.x * blockDim.x / 32;
-    double dotAcc = 0;
     // the loop bound is uniform across a warp, so every lane reaches the shuffles
     for (int base = (gid / 32) * RPW; base < nv; base += nWarps * RPW) {
         int row = base + grp;
@@ -92,27 +87,9 @@ __global__ void spmvKernel(int nv, const int* rowPtr, const int* col, const MT* 
             VT xv[3] = {x[3 * row], x[3 * row + 1], x[3 * row + 2]};
             const double* D = diagExtra + 9 * row;
             for (int q = 0; q < 3; ++q) acc[q] += (VT)(D[3 * q] * (double)xv[0] + D[3 * q + 1] * (double)xv[1] + D[3 * q + 2] * (double)xv[2]);
-            for (int q = 0; q < 3; ++q) {
-                y[3 * row + q] = acc[q];
-                dotAcc += (double)xv[q] * (double)acc[q];
-            }
+            for (int q = 0; q < 3; ++q) y[3 * row + q] = acc[q];
         }
     }
-    if (partial) {
-        double s = blockReduce(dotAcc, AddOp(), 0.0);
-        if (threadIdx.x == 0) partial[blockIdx.x] = s;
-    }
-}
-
-__device__ __forceinline__ double sumPartials(const double* p, int n) {
-    // every block sums the partials in the same order (deterministic)
-    __shared__ double sh;
-    double v = 0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) v += p[i];
-    v = blockReduce(v, AddOp(), 0.0);
-    if (threadIdx.x == 0) sh = v;
-    __syncthreads();
-    return sh;
 }
 
 // block-Jacobi inverse of the assembled diagonal blocks
@@ -148,85 +125,6 @@ __device__ __forceinline__ void applyDinv(const double* Dinv, const VT* r, VT* z
     z[3 * v] = (VT)(D[0] * r0 + D[1] * r1 + D[2] * r2);
     z[3 * v + 1] = (VT)(D[3] * r0 + D[4] * r1 + D[5] * r2);
     z[3 * v + 2] = (VT)(D[6] * r0 + D[7] * r1 + D[8] * r2);
-}
-
-// scal layout: 0 rz, 1 beta, 2 thr, 3 rr, 4 iterations, 6 rhs2
-template <class VT>
-__global__ void pcgInitKernel(int nv, const VT* b, const double* Dinv, VT* x, VT* r, VT* z, VT* p, double* part0, double* part1) {
-    double rr = 0, rz = 0;
-    CIPC_KERNEL_LOOP(v, nv) {
-        for (int q = 0; q < 3; ++q) { x[3 * v + q] = VT(0); r[3 * v + q] = b[3 * v + q]; }
-        applyDinv(Dinv, r, z, v);
-        for (int q = 0; q < 3; ++q) {
-            p[3 * v + q] = z[3 * v + q];
-            rr += (double)r[3 * v + q] * (double)r[3 * v + q];
-            rz += (double)r[3 * v + q] * (double)z[3 * v + q];
-        }
-    }
-    double a = blockReduce(rr, AddOp(), 0.0);
-    __syncthreads();
-    double c = blockReduce(rz, AddOp(), 0.0);
-    if (threadIdx.x == 0) { part0[blockIdx.x] = a; part1[blockIdx.x] = c; }
-}
-
-__global__ void pcgInitScalars(const double* part0, const double* part1, int np, double tol, double* scal, int* flag) {
-    double rr = sumPartials(part0, np);
-    double rz = sumPartials(part1, np);
-    if (threadIdx.x == 0) {
-        scal[6] = rr;
-        double thr = fmax(tol * tol * rr, 2.2250738585072014e-308);
-        scal[2] = thr;
-        scal[3] = rr;
-        scal[0] = rz;
-        scal[4] = 0;
-        *flag = (rr == 0.0 || rr < thr) ? 1 : 0;
-    }
-}
-
-// x += a p ; r -= a Ap ; z = M r ; partials of r.r and r.z
-template <class VT>
-__global__ void pcgUpdateKernel(int nv, const double* pAp, int np, const double* scal, const double* Dinv, const VT* p, const VT* Ap, VT* x, VT* r,
-                                VT* z, double* partRR, double* partRZ, const int* flag) {
-    if (*flag) return;
-    VT alpha = (VT)(scal[0] / sumPartials(pAp, np));
-    double rr = 0, rz = 0;
-    CIPC_KERNEL_LOOP(v, nv) {
-        for (int q = 0; q < 3; ++q) {
-            x[3 * v + q] += alpha * p[3 * v + q];
-            r[3 * v + q] -= alpha * Ap[3 * v + q];
-        }
-        applyDinv(Dinv, r, z, v);
-        for (int q = 0; q < 3; ++q) {
-            rr += (double)r[3 * v + q] * (double)r[3 * v + q];
-            rz += (double)r[3 * v + q] * (double)z[3 * v + q];
-        }
-    }
-    double a = blockReduce(rr, AddOp(), 0.0);
-    __syncthreads();
-    double c = blockReduce(rz, AddOp(), 0.0);
-    if (threadIdx.x == 0) { partRR[blockIdx.x] = a; partRZ[blockIdx.x] = c; }
-}
-
-// scalar step: convergence test, beta; one block.
-__global__ void pcgScalarKernel(const double* partRR, const double* partRZ, int np, double* scal, int* flag, int maxIter) {
-    if (*flag) return;
-    double rr = sumPartials(partRR, np);
-    double rz = sumPartials(partRZ, np);
-    if (threadIdx.x == 0) {
-        scal[3] = rr;
-        if (rr < scal[2]) { *flag = 1; scal[4] += 1; return; }
-        scal[1] = rz / scal[0];  // beta
-        scal[0] = rz;
-        scal[4] += 1;
-        if (scal[4] >= maxIter) *flag = 2;
-    }
-}
-
-template <class VT>
-__global__ void pcgDirKernel(int nv, const double* scal, const VT* z, VT* p, const int* flag) {
-    if (*flag == 1) return;
-    VT beta = (VT)scal[1];
-    CIPC_KERNEL_LOOP(i, 3 * nv) p[i] = z[i] + beta * p[i];
 }
 
 __global__ void rhsKernel(int nv, const double* g, const int* btype, double* b) {
@@ -1825,19 +1723,12 @@ void buildRhs(Ctx& c) {
     CIPC_CUDA(cudaGetLastError());
 }
 
-template <class MT, class VT>
-static void spmvT(Ctx& c, const MT* val, const MT* dval, const VT* x, VT* y, double* partial, const int* flag, int nblk) {
-    bool dyn = c.nDynB > 0;
-    launch(spmvKernel<MT, VT>, nblk, VB, 0, c.s, c.nv, c.rowPtr, c.colIdx, val, dyn ? c.dynRowStart.p : nullptr, dyn ? c.dynRowEnd.p : nullptr,
-           dyn ? c.dynCol.p : nullptr, dval, c.diagExtra, x, y, partial, flag);
-}
-
-static int spmvBlocks(Ctx& c) { return std::max(1, std::min((c.nv * GROUP + VB - 1) / VB, MAXPART)); }
-
-void spmv(Ctx& c, const double* x, double* y) {
-    if (c.mixed) spmvT<float, double>(c, c.valF, c.dynBF, x, y, nullptr, nullptr, spmvBlocks(c));
-    else spmvT<double, double>(c, c.valD, c.dynBD, x, y, nullptr, nullptr, spmvBlocks(c));
-    CIPC_CUDA(cudaGetLastError());
+// y = A x
+template <class MT>
+static void spmv(Ctx& c, const MT* val, const MT* dval, const double* x, double* y) {
+    const bool dyn = c.nDynB > 0;
+    launch(spmvKernel<MT, double>, std::max(1, std::min((c.nv * GROUP + VB - 1) / VB, MAXPART)), VB, 0, c.s, c.nv, c.rowPtr, c.colIdx, val,
+           dyn ? c.dynRowStart.p : nullptr, dyn ? c.dynRowEnd.p : nullptr, dyn ? c.dynCol.p : nullptr, dval, c.diagExtra, x, y);
 }
 
 static void computeDinv(Ctx& c) {
@@ -1850,45 +1741,6 @@ static void computeDinv(Ctx& c) {
     else
         launch(dinvKernel<double>, vecBlocks(nv), VB, 0, c.s, nv, c.diagSlot, c.valD, dyn ? c.dynRowStart.p : nullptr, dyn ? c.dynRowEnd.p : nullptr,
                dyn ? c.dynCol.p : nullptr, c.dynBD, c.diagExtra, c.Dinv);
-}
-
-// PCG on A x = b with vectors of type VT and blocks of type MT.  Returns the
-// iteration count; *relRes gets sqrt(rr/rhs2) of the last recursive residual.
-template <class MT, class VT>
-static int runPcg(Ctx& c, const MT* val, const MT* dval, const VT* b, VT* x, VT* r, VT* z, VT* p, VT* Ap, double tol, int maxIter,
-                  int& flagOut, double& relRes) {
-    int nv = c.nv;
-    int vb = vecBlocks(nv), sb = spmvBlocks(c);
-    double* partA = c.red.p;
-    double* partB = c.red.p + MAXPART;
-    double* partC = c.red.p + 2 * MAXPART;
-    int* flag = c.counters.p + 10;
-    launch(pcgInitKernel<VT>, vb, VB, 0, c.s, nv, b, c.Dinv, x, r, z, p, partA, partB);
-    launch(pcgInitScalars, 1, VB, 0, c.s, partA, partB, vb, tol, c.scal, flag);
-    CIPC_CUDA(cudaGetLastError());
-    const int chunk = 16;
-    int it = 0;
-    int hflag = 0;
-    double hs[8];
-    while (true) {
-        for (int k = 0; k < chunk; ++k) {
-            profBegin(c, PROF_SPMV);
-            spmvT<MT, VT>(c, val, dval, p, Ap, partC, flag, sb);
-            profEnd(c, PROF_SPMV);
-            launch(pcgUpdateKernel<VT>, vb, VB, 0, c.s, nv, partC, sb, c.scal, c.Dinv, p, Ap, x, r, z, partA, partB, flag);
-            launch(pcgScalarKernel, 1, VB, 0, c.s, partA, partB, vb, c.scal, flag, maxIter);
-            launch(pcgDirKernel<VT>, vb, VB, 0, c.s, nv, c.scal, z, p, flag);
-        }
-        CIPC_CUDA(cudaGetLastError());
-        CIPC_CUDA(cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, c.s));
-        CIPC_CUDA(cudaMemcpyAsync(hs, c.scal.p, 8 * sizeof(double), cudaMemcpyDeviceToHost, c.s));
-        hostSync(c);
-        it = (int)hs[4];
-        if (hflag) break;
-    }
-    flagOut = hflag;
-    relRes = hs[6] > 0 ? std::sqrt(hs[3] / hs[6]) : 0.0;
-    return it;
 }
 
 constexpr int PMAX = 1024;  // max blocks of the persistent PCG
@@ -2094,17 +1946,12 @@ static void launchPersistent(Ctx& c, PcgArgs<MT, VT>& a, int smCount, bool class
 template <class MT, class VT>
 static int runPcgPersistent(Ctx& c, const MT* val, const MT* dval, const VT* b, VT* x, VT* r, VT* z, VT* p, VT* Ap, double tol, int maxIter,
                             int& flagOut, double& relRes, bool learned = false, bool classic = false) {
-    static int smCount = 0, coop = -1;
-    if (coop < 0) {
-        int dev = 0;
+    static const int smCount = [] {
+        int dev = 0, sms = 0;
         CIPC_CUDA(cudaGetDevice(&dev));
-        CIPC_CUDA(cudaDeviceGetAttribute(&smCount, cudaDevAttrMultiProcessorCount, dev));
-        CIPC_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    }
-    if (!coop) {
-        if (learned) throw std::runtime_error("the learned preconditioner needs cooperative launch support");
-        return runPcg<MT, VT>(c, val, dval, b, x, r, z, p, Ap, tol, maxIter, flagOut, relRes);
-    }
+        CIPC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        return sms;
+    }();
     bool dyn = c.nDynB > 0;
     PcgArgs<MT, VT> a;
     a.nv = c.nv; a.rowPtr = c.rowPtr; a.col = c.colIdx; a.val = val;
@@ -2171,8 +2018,8 @@ static double trueResidual2(Ctx& c) {
     int nv = c.nv, n3 = 3 * nv;
     c.rF.reserve(n3);
     double* part = c.red.p + 3 * MAXPART;
-    if (c.mixed) spmvT<float, double>(c, c.valF, c.dynBF, c.sol.p, c.Ap.p, nullptr, nullptr, spmvBlocks(c));
-    else spmvT<double, double>(c, c.valD, c.dynBD, c.sol.p, c.Ap.p, nullptr, nullptr, spmvBlocks(c));
+    if (c.mixed) spmv<float>(c, c.valF, c.dynBF, c.sol.p, c.Ap.p);
+    else spmv<double>(c, c.valD, c.dynBD, c.sol.p, c.Ap.p);
     int nb = vecBlocks(nv);
     launch(residualKernel, nb, VB, 0, c.s, n3, c.rhs.p, c.Ap.p, c.r.p, c.rF.p, part);
     return deviceSum(c, part, nb);
@@ -2235,7 +2082,7 @@ static int pcgSolve64(Ctx& c) {
 static double mixedResidual(Ctx& c, float* bF) {
     int nv = c.nv, n3 = 3 * nv;
     double* part = c.red.p + 3 * MAXPART;
-    spmvT<float, double>(c, c.valF, c.dynBF, c.sol.p, c.Ap.p, nullptr, nullptr, spmvBlocks(c));
+    spmv<float>(c, c.valF, c.dynBF, c.sol.p, c.Ap.p);
     int nb = vecBlocks(nv);
     launch(residualKernel, nb, VB, 0, c.s, n3, c.rhs.p, c.Ap.p, c.r.p, bF, part);
     return deviceSum(c, part, nb);
