@@ -1050,7 +1050,7 @@ void sortKeys(Ctx& c, uint64_t* keys, int n, int endBit) {
     CIPC_CUDA(cub::DeviceRadixSort::SortKeys(c.sortTmp.p, bytes, keys, c.kTmp.p, n, 0, endBit, c.s));
     CIPC_CUDA(cudaMemcpyAsync(keys, c.kTmp.p, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, c.s));
 }
-// CIPC_SETS_APART=1: sort the active sets' lists one by one, as for scenes of over 2^20 vertices
+// CIPC_SETS_APART=1: sort the active sets' lists one by one, as in scenes too large for the joint sort
 bool sortSetsApart() {
     static int v = -1;
     if (v < 0) { const char* e = std::getenv("CIPC_SETS_APART"); v = (e && *e == '1') ? 1 : 0; }
@@ -1257,14 +1257,14 @@ void buildCollisionSets(Ctx& c, bool rehash) {
             for (int k = 0; k < 6; ++k) {
                 lists.key[k] = keys[k];
                 n += cnt[k];
-                if (n > 0x7fffffff) throw std::runtime_error("the active-set candidates exceed 2^31");
                 lists.end[k] = (int)n;
             }
             // PP/PE fields hold up to nv (c2 + 1); edge pairs of the mollified list 4 type bits
             lists.faceBits = bitsFor(c.nsf); lists.edgeBits = bitsFor(c.nse); lists.vertBits = bitsFor(c.nv + 1);
             lists.tagShift = std::max(std::max(bitsFor(c.nsv) + lists.faceBits, 2 * lists.edgeBits + 4), 3 * lists.vertBits);
-            if (lists.tagShift > 61 || sortSetsApart()) {
-                // over 2^20 vertices: three vertex fields and the list's number do not fit 64 bits
+            if (lists.tagShift > 61 || n > 0x7fffffff || sortSetsApart()) {
+                // over 2^20 vertices three vertex fields and the list's number do not
+                // fit 64 bits; the lists together may hold more keys than one alone can
                 const int endBit[6] = {32 + bitsFor(c.nsv), 32 + bitsFor(c.nsv), 63, 32 + bitsFor(c.nse), 32 + bitsFor(c.nse),
                                        std::min(64, 34 + bitsFor(c.nse))};
                 for (int k = 0; k < 6; ++k) sortKeys(c, keys[k], cnt[k], endBit[k]);
