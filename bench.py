@@ -502,7 +502,9 @@ def main():
             avg_ms = r["prof_ms"] / r["nprof"]
             achieved = bytes_ / (avg_ms / 1000.0) / 1e9
             iters_per_launch = r["pcg"] / r["nprof"]
-            roof = {"kernel": "pcgPipelinedKernel (whole PCG solve, one cooperative launch)", "bound": "hbm", "achieved": achieved,
+            # rows beyond one block of 128 per SM are streamed in tiles
+            single = nv <= 128 * torch.cuda.get_device_properties(0).multi_processor_count
+            roof = {"kernel": ("pcgPipelinedKernel" if single else "pcgStreamKernel") + " (whole PCG solve, one cooperative launch)", "bound": "hbm", "achieved": achieved,
                     "peak": peak, "peak_source": peak_kind, "unit": "GB/s", "frac": achieved / peak, "traffic": ncu_traffic(workload(args)),
                     "algorithmic_bytes_per_launch": bytes_, "bytes_per_iteration": per_it, "launches": r["nprof"],
                     "mean_launch_us": 1000 * avg_ms, "us_per_iteration": 1000 * avg_ms / max(1e-9, iters_per_launch),
