@@ -1,14 +1,15 @@
 // Broad phase and step bounds on the GPU.
 //
-// * LBVH build: primitive boxes -> scene box -> 30-bit Morton keys with the
-//   primitive id in the low word -> radix sort -> Karras internal nodes ->
-//   bottom-up boxes (first-arrival flags).  Topology follows
-//   CPULinearBVH::build, CPU IPC/LBVH.cpp:163-250.
-// * Active sets: one thread per query traverses the tree with the inclusive
-//   overlaps(gap) test (LBVH.cpp:157-161), applies the collider / incidence
-//   filters of SpatialHash::calculateActivateSet
-//   (CPU IPC/CollisionBroadPhase.cpp:765-1059), classifies and emits 64-bit
-//   pair keys.  Keys are radix-sorted, so every list comes out in the
+// * LBVH build, faces and edges by the same launches: primitive boxes and scene
+//   box -> 30-bit Morton keys with the primitive id in the low word -> one radix
+//   sort -> Karras internal nodes -> bottom-up boxes (arrival flags).  Topology
+//   follows CPULinearBVH::build, CPU IPC/LBVH.cpp:163-250.
+// * Active sets: a warp walks the tree for 32 queries with one shared stack, by
+//   the inclusive overlaps(gap) test (LBVH.cpp:157-161), applies the collider /
+//   incidence filters of SpatialHash::calculateActivateSet
+//   (CPU IPC/CollisionBroadPhase.cpp:765-1059) and emits candidate pairs; one
+//   thread per candidate classifies it and emits 64-bit pair keys.  Keys are
+//   radix-sorted together, so every list comes out in the
 //   reference's order (query ascending, then primitive ascending); PP/PE
 //   duplicates are merged by sort + run-length encoding, the job of the
 //   reference's std::map.
